@@ -141,70 +141,75 @@ WR_MHD double wr_fixed_to_double(int64_t hi, uint64_t lo, int q) {
 // exact remainder correction of the quotient (the Newton-Raphson-based division of
 // J.-M. Muller et al., Handbook of Floating-Point Arithmetic, 2nd ed., Birkhauser
 // 2018), carried out in fixed point.  Normal operands with a normal quotient take
-// the integer path: a float reciprocal of the divisor's top 24 bits, two
-// fixed-point Newton steps (Q63), a 54-bit quotient, an exact remainder check and
-// round-to-nearest-even.
-// Everything else (zeros, subnormals, inf/NaN, overflow/underflow) uses a / b.
-// On GB300 this keeps divisions off the FP64 pipe (a native double division
-// issues about eight FP64 instructions).  wr_div_int (below) is
+// the integer path; everything else (zeros, subnormals, inf/NaN, overflow/underflow)
+// uses a / b.  On GB300 this keeps divisions off the FP64 pipe (a native double
+// division issues about eight FP64 instructions).  wr_div_int (below) is
 // wr_div_finish(a, b, wr_div_recip(b)).
+//
+// What bounds it on the GPU is its instruction count and serial length: a lone warp
+// pays 4-5 cycles per instruction, and 16 warps share one instruction cache.  So the
+// first Newton step works on 32-bit halves, every estimate stays below the exact
+// value, and the quotient then needs one correction.
 
-// The divisor's part of wr_div_int: Y ~ 1/b_m in Q63 (b_m = b's significand in
-// [1, 2)) from a float seed and two fixed-point Newton steps.  Any value for a
-// zero, subnormal, infinite or NaN b (wr_div_finish then divides by a / b).  A
-// quotient needs only wr_div_finish with this Y, so several divisions by one b
-// share it.
+// The divisor's part: Y in [t (1 - 2^-59), t], t = 2^64 / b_m, for b's significand b_m
+// in [1, 2) (2^64 - 1 at most).  With B = b_m 2^63 and b' = floor(B / 2^32) + 1:
+//   y0 = 2^63 / b' (1 - d), 2^-22 < d < 2^-20.4: a float reciprocal (1 ulp) of the
+//        divisor's top 32 bits, lowered by 2^-21;
+//   y1 = y0 2^32 (1 + d) from e = 2^63 - b' y0 in (0, 2^43): below 2^95 / b' by less
+//        than 2^-40 relative, so below t by less than 2^-30.9;
+//   Y  = y1 (1 + d1), d1 = 1 - b_m y1 / 2^64 < 2^-30.9, every truncation downwards:
+//        d1^2 + 2^-62 + 2^-63 + 2^-63 < 2^-60 below t.
+// Any value for a zero, subnormal, infinite or NaN b (wr_div_finish then divides by
+// a / b).  A quotient needs only wr_div_finish with this Y, so several divisions by
+// one b share it.
 WR_MHD uint64_t wr_div_recip(double b) {
-    const uint64_t ub = wr_bits(b);
-    const uint64_t mb = (ub & 0x000fffffffffffffULL) | 0x0010000000000000ULL;
-    const float bf = static_cast<float>(static_cast<uint32_t>(mb >> 29));  // exact, 24 bits
+    const uint64_t B = (wr_bits(b) | 0x0010000000000000ULL) << 11;
+    const uint32_t bh = static_cast<uint32_t>(B >> 32);
+    const float bf = static_cast<float>(bh);
+    float rf;
 #if defined(__CUDA_ARCH__)
-    const float rf = __frcp_rn(bf);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(bf));
 #else
-    const float rf = 1.0f / bf;
+    rf = 1.0f / bf;
 #endif
-    uint64_t Y = static_cast<uint64_t>(static_cast<uint32_t>(rf * 18014398509481984.0f)) << 32;
-    const uint64_t B = mb << 10;  // b_m * 2^62
-#pragma unroll
-    for (int it = 0; it < 2; ++it) {
-        const int64_t e = static_cast<int64_t>(0x2000000000000000ULL - wr_umulhi(B, Y));  // (1 - b y) * 2^61
-        const uint64_t c = e >= 0 ? wr_umulhi(Y, static_cast<uint64_t>(e)) : 0 - wr_umulhi(Y, static_cast<uint64_t>(-e));
-        Y += c << 3;
-    }
-    return Y;
+    const uint32_t y0 = static_cast<uint32_t>(rf * 9223367638808264704.0f);  // 2^63 (1 - 2^-21)
+    const uint64_t e = 0x8000000000000000ULL - (static_cast<uint64_t>(bh) * y0 + y0);
+    const uint64_t c = static_cast<uint64_t>(static_cast<uint32_t>(e >> 11)) * y0;
+    const uint64_t y1 = (static_cast<uint64_t>(y0) << 32) + (c >> 20);
+    const uint64_t e1 = 0x7fffffffffffffffULL - wr_umulhi(B, y1);
+    const uint64_t c1 = static_cast<uint64_t>(static_cast<uint32_t>(e1 >> 1)) * static_cast<uint32_t>(y1 >> 32);
+    return y1 + (c1 >> 30);
 }
 
-// a / b given Y = wr_div_recip(b): a 54-bit quotient Q ~ floor(a_m * 2^(53+adj) /
-// b_m), its exact remainder, at most two corrections each way, round to nearest
-// even.  Operands or quotients outside the normal range divide by a / b.
+// a / b given Y = wr_div_recip(b): the quotient's 54 bits Q = floor(a_m 2^(53+adj) /
+// b_m) from the estimate with Y (Y's error moves it by less than 2^-5, so it is Q or
+// Q - 1), its exact remainder, round to nearest even.  Operands or quotients outside
+// the normal range divide by a / b; one exit for all of them, since a copy of the
+// native division costs the kernels' instruction cache two kilobytes.
 WR_MHD double wr_div_finish(double a, double b, uint64_t Y) {
     const uint64_t ua = wr_bits(a), ub = wr_bits(b);
     const uint32_t ea = static_cast<uint32_t>(ua >> 52) & 0x7ff;
     const uint32_t eb = static_cast<uint32_t>(ub >> 52) & 0x7ff;
-    if (ea - 1u >= 2046u || eb - 1u >= 2046u) return a / b;
     const uint64_t ma = (ua & 0x000fffffffffffffULL) | 0x0010000000000000ULL;
     const uint64_t mb = (ub & 0x000fffffffffffffULL) | 0x0010000000000000ULL;
     const int adj = ma < mb ? 1 : 0;
-    const int be = static_cast<int>(ea) - static_cast<int>(eb) - adj + 1023;
-    if (be < 1 || be > 2046) return a / b;
-    uint64_t Q = wr_umulhi(ma << (2 + adj), Y);
-    int64_t R = static_cast<int64_t>((ma << (53 + adj)) - Q * mb);
-    const int64_t smb = static_cast<int64_t>(mb);
-    if (R < 0) { Q -= 1; R += smb; }
-    if (R < 0) { Q -= 1; R += smb; }
-    if (R >= smb) { Q += 1; R -= smb; }
-    if (R >= smb) { Q += 1; R -= smb; }
-    uint64_t mant = Q >> 1;
-    const bool up = (Q & 1) && (R != 0 || (mant & 1));
-    mant += up ? 1 : 0;
-    int e2 = be;
-    if (mant >> 53) {
-        mant >>= 1;
-        e2 += 1;
-        if (e2 > 2046) return a / b;
+    const int be = static_cast<int>(ea) - static_cast<int>(eb) - adj + 1022;
+    if (ea - 1u < 2046u && eb - 1u < 2046u && static_cast<unsigned>(be) < 2046u) {
+        const uint64_t m = ma << adj;
+        uint64_t Q = wr_umulhi(m << 1, Y);
+        uint64_t R = (m << 53) - Q * mb;
+        const bool more = R >= mb;
+        Q += more ? 1 : 0;
+        R -= more ? mb : 0;
+        const uint64_t mant = Q >> 1;
+        const uint64_t up = (Q & 1) & ((R != 0 ? 1 : 0) | (mant & 1));
+        // mant has its leading bit 2^52, which raises the exponent field by one, and
+        // rounding up to 2^53 by two: the next binade's first number (infinity at the
+        // top, which a / b gives)
+        const uint64_t r = (static_cast<uint64_t>(static_cast<uint32_t>(be)) << 52) + mant + up;
+        return wr_from_bits(r | ((ua ^ ub) & 0x8000000000000000ULL));
     }
-    return wr_from_bits(((ua ^ ub) & 0x8000000000000000ULL) | (static_cast<uint64_t>(e2) << 52) |
-                        (mant & 0x000fffffffffffffULL));
+    return a / b;
 }
 
 WR_MHD double wr_div_int(double a, double b) { return wr_div_finish(a, b, wr_div_recip(b)); }
@@ -357,6 +362,9 @@ WR_MHD double wr_cbrt(double x) {
     const uint64_t b = wr_bits(a);
     double y = wr_from_bits(b / 3 + 0x2a9f800000000000ULL);
     const double third = 1.0 / 3.0;
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1  // one copy of the division: instruction-cache space
+#endif
     for (int it = 0; it < 4; ++it) y = y + (wr_div_int(a, y * y) - y) * third;
     y = y * scale;
     return (u >> 63) ? -y : y;
