@@ -186,8 +186,10 @@ int wr_set_profiling(wr_ctx* ctx, int on);
  *      exp/log, stage combination, error norm, controller and EOS stay FP64
  *   4  one lane per cell, 384 lanes per SM (1 block), matrix in global memory
  *   5  cooperative: 8 lanes per cell (4 cells per warp), 9 warps per SM
- *   6  cooperative: 16 lanes per cell (2 cells per warp), 16 warps per SM (default)
+ *   6  cooperative: 16 lanes per cell (2 cells per warp), 16 warps per SM
  *   7  cooperative: 32 lanes per cell (1 cell per warp), 16 warps per SM
+ * A new context uses 7 up to 16 cells per SM (2,432 cells on 152 SMs: every cell has a
+ * warp at once, and the shorter attempt decides) and 6 beyond.
  * The cooperative advance evaluates one cell's network, LU factorisation and
  * triangular solves with a group of lanes (generated vector programs, a
  * warp-cooperative LU with shuffle pivot search, shared-memory matrices).

@@ -18,19 +18,18 @@ struct Tab {
     static constexpr int kNV = cp::kNV;
     static constexpr int kNR = cp::kNR;
     static constexpr int kNF = cp::kNF;
-    static constexpr int kJSteps = cp::kJRHSSteps;
-    static constexpr int kRSteps = cp::kRHSSteps;
-    static __device__ __forceinline__ const ulonglong2* jprog() { return cp::kJRHSProg; }
-    static __device__ __forceinline__ const uint64_t* jlit() { return cp::kJRHSLit; }
-    static __device__ __forceinline__ const ulonglong2* rprog() { return cp::kRHSProg; }
-    static __device__ __forceinline__ const uint64_t* rlit() { return cp::kRHSLit; }
-    static __device__ __forceinline__ const uint16_t* jout() { return cp::kJRHSOut; }
-    static __device__ __forceinline__ const uint16_t* jac() { return cp::kJRHSJac; }
-    static __device__ __forceinline__ const uint16_t* rout() { return cp::kRHSOut; }
+    static constexpr int kRegimes = cp::kRegimes;
     static __device__ __forceinline__ const uint64_t* vconst() { return cp::kVConst; }
     static __device__ __forceinline__ const ulonglong2* vfun() { return cp::kVFun; }
+    static __device__ __forceinline__ const ulonglong2* prog() { return cp::kProg; }
+    static __device__ __forceinline__ const uint64_t* lit() { return cp::kLit; }
+    static __device__ __forceinline__ uint32_t ctl(int i) { return cp::kCtl[i]; }
+    static __device__ __forceinline__ int first(int w) { return cp::kProgStep[w][0]; }
+    static __device__ __forceinline__ int steps(int w) { return cp::kProgStep[w][1]; }
+    static __device__ __forceinline__ uint64_t regime(int k, int i) { return cp::kRegimeT[k][i]; }
+    static __device__ __forceinline__ const uint16_t* out(int w) { return cp::kOut[w]; }
+    static __device__ __forceinline__ const uint16_t* jac(int r) { return cp::kJac[r]; }
 };
-static_assert(Tab::kJSteps % 4 == 0 && Tab::kRSteps % 4 == 0, "programs are padded to groups of four steps");
 static_assert(coop::kRes + Tab::kNR + Tab::kNF <= Tab::kNV, "reserved constants lie inside the slot array");
 
 constexpr int kG = WR_COOP_G;

@@ -51,7 +51,7 @@ struct wr_ctx {
     int math = WR_MATH_PORTABLE;
     int advance_blocks = 0;
     int sms = 1;
-    int variant = kDefaultVariant;  // the cooperative advance, 16 lanes per cell
+    int variant = kDefaultVariant;  // wr_create: the cooperative advance, 32 or 16 lanes per cell
     cudaStream_t stream = nullptr;
     DevState s{};
     void* state_buf = nullptr;
@@ -479,6 +479,7 @@ int wr_create_batch(int num_grids, const int* cells_per_grid, int device, int ma
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     ctx->sms = sms > 0 ? sms : 1;
     ctx->advance_blocks = ctx->sms;
+    ctx->variant = default_variant(num_cells, ctx->sms);
     size_t nslots = 0;  // lane slots of the largest configuration
     for (const AdvanceShape& sh : kAdvanceShapes) {
         const size_t slots = static_cast<size_t>(ctx->sms) * sh.blocks_per_sm * sh.threads;

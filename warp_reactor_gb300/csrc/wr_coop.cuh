@@ -51,16 +51,20 @@ namespace coop {
 
 enum { C_NONE = 0, C_FMA = 1, C_EXP = 2, C_LOG = 3, C_SQRT = 4, C_DIV = 5 };
 enum { I_SEL = 0, I_LE = 1, I_LT = 2, I_SGN = 3 };
-// flags in the low three bits of the 16-bit byte-offset fields of a step
+// control byte of a step: class | CTL_INT (it has integer nodes) | CTL_SPECIAL (they
+// include comparisons or sign operations) | CTL_FLUSH (its main results are stored in
+// the step itself)
+enum : uint32_t { CTL_CLASS = 7u, CTL_INT = 8u, CTL_SPECIAL = 16u, CTL_FLUSH = 32u };
+// flags in the low three bits of the 16-bit destination fields of a step
 enum : uint32_t {
-    FL_NEG = 1u, FL_ABS = 2u, FL_SWAP = 4u,  // X, Y: argument modifiers; Y: divide V[Y] ^ L by V[X]
-    FL_INT = 1u, FL_SPECIAL = 2u,            // Z: integer nodes / comparisons or sign ops in the step
-    FL_SABS = 4u                             // integer destination of I_SGN: clear the sign (else flip)
+    DV_NEG = 1u, DV_ABS = 2u, DV_SWAP = 4u,  // D: argument modifiers; divide V[Y] ^ L by V[X]
+    FL_SABS = 4u                             // D2 of I_SGN: clear the sign (else flip)
 };
 constexpr int kE = 0;        // iteration matrix slots [0, 225)
 constexpr int kY = 225;      // program inputs y[0..14]
 constexpr int kRes = 240;    // reserved constants [240, 240 + Tab::kNR + Tab::kNF)
 constexpr uint32_t kOff = 0xfff8u;
+constexpr unsigned kWarp = 0xffffffffu;
 constexpr uint64_t kSign = 0x8000000000000000ULL;
 constexpr uint64_t kAbs = 0x7fffffffffffffffULL;
 constexpr uint64_t kInfBits = 0x7ff0000000000000ULL;
@@ -87,14 +91,10 @@ __device__ __forceinline__ uint64_t lds64(uint32_t addr) {
 __device__ __forceinline__ void sts64(uint32_t addr, uint64_t v) {
     asm volatile("st.shared.b64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
 }
-__device__ __forceinline__ void group_sync(unsigned gmask) {
-    asm volatile("bar.warp.sync %0;" ::"r"(gmask) : "memory");
-}
-// sign modifiers of an exp/log/sqrt/div argument (abs, then negate)
-__device__ __forceinline__ uint64_t modify(uint64_t v, uint32_t fl) {
-    v = (fl & FL_ABS) ? (v & kAbs) : v;
-    return (fl & FL_NEG) ? (v ^ kSign) : v;
-}
+// base + the low (high) 16-bit field of w: one integer dot-product instruction
+// instead of a mask (shift) and an add
+__device__ __forceinline__ uint32_t addr_lo(uint32_t w, uint32_t base) { return __dp2a_lo(w, 0x0001u, base); }
+__device__ __forceinline__ uint32_t addr_hi(uint32_t w, uint32_t base) { return __dp2a_lo(w, 0x0100u, base); }
 
 // IEEE a <= b and a < b on bit patterns: false when either is NaN, -0 == +0
 __device__ __forceinline__ uint64_t ble(uint64_t a, uint64_t b) {
@@ -114,98 +114,160 @@ __device__ __forceinline__ uint64_t blt(uint64_t a, uint64_t b) {
     return (!nan && !zero && (sa != sb ? sa : same)) ? 1ULL : 0ULL;
 }
 
-// Transcendental steps call one out-of-line copy each, so the interpreter loop
-// stays small (CUDA's own functions inside for CudaMath).
+// Transcendentals are one out-of-line copy each (CUDA's own functions inside for
+// CudaMath), as are the solve and the evaluation: the attempt's code has to stay near
+// the instruction cache's size, with 16 warps in different phases of it.
 template <class M>
 struct StepMath {
     static __device__ __noinline__ double exp(double x) { return M::exp(x); }
     static __device__ __noinline__ double log(double x) { return M::log(x); }
     static __device__ __noinline__ double sqrt(double x) { return M::sqrt(x); }
+    static __device__ __noinline__ double cbrt(double x) { return M::cbrt(x); }
 };
 
-// One step of one lane.  e.x: main word X | Y | Z | D (16-bit byte offsets into
-// the cell's slot array at shared address vb, flags in their low three bits);
-// e.y: integer word A | B | C | D2; lit: the lane's literal, XOR-ed into V[Y].
-// An FMA step's operand offsets carry no flags (the generator guarantees it), so
-// they are added to vb as they are.
+// main result of a division, exp, log or sqrt step: x = V[X], y = V[Y] ^ L, fl the
+// modifier flags of D
 template <class M>
-__device__ __forceinline__ void exec_step(const ulonglong2 e, const uint64_t lit, uint32_t vb) {
-    const uint32_t w0 = static_cast<uint32_t>(e.x), w1 = static_cast<uint32_t>(e.x >> 32);
-    const uint32_t cls = (w1 >> 16) & 7u;
-    const uint32_t dst = vb + ((w1 >> 16) & kOff);
-    if (cls == C_FMA) {
-        const double a = dbl(lds64(vb + (w0 & 0xffffu)));
-        const double b = dbl(lds64(vb + (w0 >> 16)) ^ lit);
-        const double c = dbl(lds64(vb + (w1 & kOff)));
-        sts64(dst, bits(__fma_rn(a, b, c)));
-    } else if (cls != C_NONE) {
-        const uint32_t yf = w0 >> 16;
-        const uint64_t y = modify(lds64(vb + (yf & kOff)) ^ lit, yf);
-        double r;
-        if (cls == C_DIV) {
-            const uint64_t x = modify(lds64(vb + (w0 & kOff)), w0);
-            const bool sw = (yf & FL_SWAP) != 0;
-            r = ddiv(dbl(sw ? y : x), dbl(sw ? x : y));
-        } else if (cls == C_EXP) {
-            r = StepMath<M>::exp(dbl(y));
-        } else if (cls == C_LOG) {
-            r = StepMath<M>::log(dbl(y));
-        } else {
-            r = StepMath<M>::sqrt(dbl(y));
-        }
-        sts64(dst, bits(r));
+__device__ __noinline__ uint64_t slow_step(uint32_t cls, uint64_t x, uint64_t y, uint32_t fl) {
+    if (cls == C_DIV) {
+        x = (fl & DV_ABS) ? (x & kAbs) : x;
+        x = (fl & DV_NEG) ? (x ^ kSign) : x;
+        const bool sw = (fl & DV_SWAP) != 0;
+        return bits(ddiv(dbl(sw ? y : x), dbl(sw ? x : y)));
     }
-    if (w1 & FL_INT) {  // the step carries integer nodes (uniform over the warp)
-        const uint32_t i0 = static_cast<uint32_t>(e.y), i1 = static_cast<uint32_t>(e.y >> 32);
-        const uint64_t A = lds64(vb + (i0 & 0xffffu));
-        const uint64_t B = lds64(vb + (i0 >> 16));
-        const uint64_t C = lds64(vb + (i1 & 0xffffu));
-        uint64_t r = A != 0 ? B : C;
-        if (w1 & FL_SPECIAL) {  // comparisons or sign operations (uniform over the warp)
-            const uint32_t iop = (i1 >> 16) & 3u;
-            r = iop == I_LE ? ble(A, B) : r;
-            r = iop == I_LT ? blt(A, B) : r;
-            r = iop == I_SGN ? (((i1 >> 16) & FL_SABS) ? (A & kAbs) : (A ^ kSign)) : r;
-        }
-        sts64(vb + ((i1 >> 16) & kOff), r);
-    }
+    y = (fl & DV_ABS) ? (y & kAbs) : y;
+    y = (fl & DV_NEG) ? (y ^ kSign) : y;
+    if (cls == C_EXP) return bits(StepMath<M>::exp(dbl(y)));
+    if (cls == C_LOG) return bits(StepMath<M>::log(dbl(y)));
+    return bits(StepMath<M>::sqrt(dbl(y)));
 }
 
-// One generated program on the group's cell: the steps' words per lane; the group
-// synchronises after every step.  One out-of-line copy serves every call site (the
-// instruction cache holds one loop).  The step count is a multiple of four and the
-// tables carry four idle steps more, so the loop runs four steps per iteration and
-// loads each step's words four steps before it executes them (the tables, ~100-200
-// KB per G, live mostly in L2: shared memory takes most of L1).
-template <class M, int G>
-__device__ __noinline__ void run_prog(const ulonglong2* __restrict__ prog, const uint64_t* __restrict__ lits,
-                                      int nsteps, int gl, uint64_t* V, unsigned gmask) {
+// the integer node of a step: iw = A | B | C | D2
+static __device__ __noinline__ void int_step(uint32_t c, uint64_t iw, uint32_t vb) {
+    const uint32_t i0 = static_cast<uint32_t>(iw), i1 = static_cast<uint32_t>(iw >> 32);
+    const uint64_t A = lds64(addr_lo(i0, vb)), B = lds64(addr_hi(i0, vb)), C = lds64(addr_lo(i1, vb));
+    uint64_t v = A != 0 ? B : C;
+    if (c & CTL_SPECIAL) {  // comparisons or sign operations
+        const uint32_t d2 = i1 >> 16, iop = d2 & 3u;
+        v = iop == I_LE ? ble(A, B) : v;
+        v = iop == I_LT ? blt(A, B) : v;
+        v = iop == I_SGN ? ((d2 & FL_SABS) ? (A & kAbs) : (A ^ kSign)) : v;
+    }
+    sts64(addr_hi(i1, vb) & ~7u, v);
+}
+
+// One generated program on the warp's cells, every lane in step.
+//
+// Step words of one lane: e.x = X | Y | Z | D and e.y = A | B | C | D2, 16-bit byte
+// offsets into the cell's slot array at shared address vb (flags in the low bits of
+// D and D2), and the lane's literal, XOR-ed into V[Y].  Main node V[D] =
+// fma(V[X], V[Y] ^ L, V[Z]) or the step's other class; integer node V[D2] =
+// V[A] != 0 ? V[B] : V[C] or a comparison or sign operation.  A step's class is the
+// same for all lanes and comes from a control byte in constant memory, so its tests
+// are uniform branches.
+//
+// A lone warp needs ~500 cycles for an FMA step when each step loads, computes,
+// stores and synchronises before the next begins: decode, 30 cycles of shared
+// memory, 64+ of FP64, store and barrier in one chain.  So the steps overlap: step s
+// issues its FP64 instruction on operands loaded during step s - 1, then the
+// results of step s - 1 are stored and the operands of step s + 1 loaded while it
+// runs.  The generator keeps a main result MAIN_DELAY = 2 steps from its first use
+// (or marks its step CTL_FLUSH), an integer node's INT_DELAY = 1.
+//
+// The loop runs four steps per iteration and loads the words of the next four at its
+// top, in one batch.  A load per step, four
+// steps ahead, made every step wait for the L2 latency of the newest one, since the
+// few scoreboards of a warp are shared with the operand loads (Jacobian program at 16
+// lanes, CUDA math, 16 warps in one block: 345 k cycles a run, 264 k in batches; a
+// lone warp 211 k and 173 k).  The tables carry four idle steps past the end.  One
+// out-of-line copy serves every call site: the instruction cache holds one loop.
+__device__ __forceinline__ ulonglong2 ld_words(const ulonglong2* p) {
+    ulonglong2 v;
+    asm volatile("ld.global.nc.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint64_t ld_lit(const uint64_t* p) {
+    uint64_t v;
+    asm volatile("ld.global.nc.u64 %0, [%1];" : "=l"(v) : "l"(p));
+    return v;
+}
+template <int G>
+struct StepWords {
+    ulonglong2 e[4];
+    uint64_t l[4];
+    __device__ __forceinline__ void load(const ulonglong2* p, const uint64_t* q) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) e[k] = ld_words(p + k * G);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) l[k] = ld_lit(q + k * G);
+    }
+};
+template <class M, int G, class Tab>
+__device__ __noinline__ void run_prog(int which, int gl, uint64_t* V) {
     const uint32_t vb = static_cast<uint32_t>(__cvta_generic_to_shared(V));
-    const ulonglong2* p = prog + gl;
-    const uint64_t* q = lits + gl;
-    ulonglong2 e0 = __ldg(p), e1 = __ldg(p + G), e2 = __ldg(p + 2 * G), e3 = __ldg(p + 3 * G);
-    uint64_t l0 = __ldg(q), l1 = __ldg(q + G), l2 = __ldg(q + 2 * G), l3 = __ldg(q + 3 * G);
+    which = __shfl_sync(kWarp, which, 0);  // uniform over the warp
+    const int first = Tab::first(which), nsteps = Tab::steps(which), ctl0 = first / 4;
+    const ulonglong2* p = Tab::prog() + first * G + gl;
+    const uint64_t* q = Tab::lit() + first * G + gl;
+    StepWords<G> a, b;
+    a.load(p, q);
+    uint64_t x, y, z;
+    auto operands = [&](const ulonglong2 e, const uint64_t l) {
+        const uint32_t w0 = static_cast<uint32_t>(e.x), w1 = static_cast<uint32_t>(e.x >> 32);
+        x = lds64(addr_lo(w0, vb));
+        y = lds64(addr_hi(w0, vb)) ^ l;
+        z = lds64(addr_lo(w1, vb));
+    };
+    operands(a.e[0], a.l[0]);
+    uint64_t res = 0;                         // the last step's main results,
+    uint32_t dst = vb + (Tab::kNV - 1) * 8;   // stored while this step's run
+    auto step = [&](const ulonglong2 e, uint32_t c, const ulonglong2 en, const uint64_t ln) {
+        const uint32_t w1 = static_cast<uint32_t>(e.x >> 32);
+        const uint32_t cls = c & CTL_CLASS;
+        uint64_t r = 0;
+        if (cls == C_FMA)
+            r = bits(__fma_rn(dbl(x), dbl(y), dbl(z)));
+        else if (cls != C_NONE)
+            r = slow_step<M>(cls, x, y, w1 >> 16);
+        if (c & CTL_INT) int_step(c, e.y, vb);
+        if (c & CTL_FLUSH) sts64(addr_hi(w1, vb) & ~7u, r);
+        sts64(dst, res);
+        __syncwarp();
+        operands(en, ln);
+        res = r;
+        dst = addr_hi(w1, vb) & ~7u;
+    };
 #pragma unroll 1
     for (int s = 0; s < nsteps; s += 4) {
+        const uint32_t c0 = Tab::ctl(ctl0 + s / 4);
         p += 4 * G;
         q += 4 * G;
-        exec_step<M>(e0, l0, vb);
-        e0 = __ldg(p);
-        l0 = __ldg(q);
-        group_sync(gmask);
-        exec_step<M>(e1, l1, vb);
-        e1 = __ldg(p + G);
-        l1 = __ldg(q + G);
-        group_sync(gmask);
-        exec_step<M>(e2, l2, vb);
-        e2 = __ldg(p + 2 * G);
-        l2 = __ldg(q + 2 * G);
-        group_sync(gmask);
-        exec_step<M>(e3, l3, vb);
-        e3 = __ldg(p + 3 * G);
-        l3 = __ldg(q + 3 * G);
-        group_sync(gmask);
+        b.load(p, q);
+        step(a.e[0], c0, a.e[1], a.l[1]);
+        step(a.e[1], c0 >> 8, a.e[2], a.l[2]);
+        step(a.e[2], c0 >> 16, a.e[3], a.l[3]);
+        step(a.e[3], c0 >> 24, b.e[0], b.l[0]);
+        a = b;
     }
+    sts64(dst, res);
+    __syncwarp();
+}
+
+// The programs of a state (Jacobian program at 16 lanes, CUDA math, a block of 16
+// warps: 285 k cycles for the general one, 238 k for a regime's; the RHS program 127 k
+// and 102 k): regime 0 is right for every state; the others are the
+// network specialised to a range of temperatures (fewer nodes, the same bits where T
+// lies in the range).  T is a result of the program itself, so the regime is a guess,
+// the cell's regime at its last evaluation, checked afterwards: the general program
+// runs again where a cell's T lies outside.  The warp's cells share one program: where
+// their guesses differ, the last regime, which spans all others.
+template <class Tab>
+__device__ __forceinline__ int regime_of(uint64_t T) {
+    int r = 0;
+#pragma unroll
+    for (int k = Tab::kRegimes - 1; k > 0; --k)
+        if (T > Tab::regime(k, 0) && T <= Tab::regime(k, 1)) r = k;
+    return r;
 }
 
 // the reserved constants of the programs into the group's slot array (once per
@@ -213,7 +275,7 @@ __device__ __noinline__ void run_prog(const ulonglong2* __restrict__ prog, const
 // here with the kernel's own functions so that they are the bits a program step
 // would compute
 template <class M, int G, class Tab>
-__device__ __forceinline__ void init_reserved(uint64_t* V, int gl, unsigned gmask) {
+__device__ __forceinline__ void init_reserved(uint64_t* V, int gl) {
     for (int i = gl; i < Tab::kNR; i += G) V[kRes + i] = Tab::vconst()[i];
     for (int i = gl; i < Tab::kNF; i += G) {
         const ulonglong2 f = Tab::vfun()[i];
@@ -221,16 +283,19 @@ __device__ __forceinline__ void init_reserved(uint64_t* V, int gl, unsigned gmas
         const double r = f.x == C_EXP ? StepMath<M>::exp(a) : f.x == C_LOG ? StepMath<M>::log(a) : StepMath<M>::sqrt(a);
         V[kRes + Tab::kNR + i] = bits(r);
     }
-    __syncwarp(gmask);
+    __syncwarp();
 }
 
 // lu_decomposition<15> (reproducer.cpp:96-151) by the G lanes of a group on the
 // matrix E[r*15 + c] in shared memory: the same pivot (first strictly largest
 // |a_ik|, a NaN diagonal keeps its row), the same row interchange, negated
-// multipliers and rank-1 update, each element the same two roundings.
+// multipliers and rank-1 update, each element the same two roundings.  The warp's
+// groups stay in step (a group with a zero pivot idles through the column), and a
+// lane updates four elements at a time: their loads and FP64 latencies overlap.
 template <int G>
-__device__ __forceinline__ int lu_coop(double* E, int gl, unsigned gmask, uint64_t& ip) {
+__device__ __forceinline__ int lu_coop(double* E, int gl, uint64_t& ip) {
     constexpr int K = (NEQ + G - 1) / G;
+    constexpr int U = 4;
     int info = 0;
     uint64_t piv = 0;
 #pragma unroll 1
@@ -251,8 +316,8 @@ __device__ __forceinline__ int lu_coop(double* E, int gl, unsigned gmask, uint64
         }
 #pragma unroll
         for (int off = G / 2; off > 0; off >>= 1) {
-            const long long ok = __shfl_xor_sync(gmask, key, off, G);
-            const int oi = __shfl_xor_sync(gmask, idx, off, G);
+            const long long ok = __shfl_xor_sync(kWarp, key, off, G);
+            const int oi = __shfl_xor_sync(kWarp, idx, off, G);
             if (ok > key || (ok == key && oi < idx)) {
                 key = ok;
                 idx = oi;
@@ -260,39 +325,60 @@ __device__ __forceinline__ int lu_coop(double* E, int gl, unsigned gmask, uint64
         }
         const int p = idx;
         piv |= static_cast<uint64_t>(p) << (4 * k);
-        if (E[p * NEQ + k] != 0.0) {
-            if (p != k) {
+        const double pivot = E[p * NEQ + k];
+        const bool nz = pivot != 0.0;
+        double rk[K], rp[K];
 #pragma unroll
-                for (int t = 0; t < K; ++t) {
-                    const int j = k + gl + t * G;
-                    if (j < NEQ) {
-                        const double tmp = E[p * NEQ + j];
-                        E[p * NEQ + j] = E[k * NEQ + j];
-                        E[k * NEQ + j] = tmp;
-                    }
-                }
-                __syncwarp(gmask);
-            }
-            const double mult = ddiv(-1.0, E[k * NEQ + k]);
+        for (int t = 0; t < K; ++t) {
+            const int j = k + gl + t * G;
+            rk[t] = j < NEQ ? E[k * NEQ + j] : 0.0;
+            rp[t] = j < NEQ ? E[p * NEQ + j] : 0.0;
+        }
+        __syncwarp();
+        if (nz && p != k) {
 #pragma unroll
             for (int t = 0; t < K; ++t) {
-                const int i = k + 1 + gl + t * G;
-                if (i < NEQ) E[i * NEQ + k] = E[i * NEQ + k] * mult;
+                const int j = k + gl + t * G;
+                if (j < NEQ) {
+                    E[p * NEQ + j] = rk[t];
+                    E[k * NEQ + j] = rp[t];
+                }
             }
-            __syncwarp(gmask);
-            const int m = NEQ - 1 - k;
-            const unsigned cm = (65536u + static_cast<unsigned>(m) - 1u) / static_cast<unsigned>(m);
+        }
+        __syncwarp();
+        if (!nz) info = k + 1;
+        const double mult = ddiv(-1.0, pivot);
+#pragma unroll
+        for (int t = 0; t < K; ++t) {
+            const int i = k + 1 + gl + t * G;
+            if (nz && i < NEQ) E[i * NEQ + k] = E[i * NEQ + k] * mult;
+        }
+        __syncwarp();
+        const int m = NEQ - 1 - k;
+        const unsigned cm = (65536u + static_cast<unsigned>(m) - 1u) / static_cast<unsigned>(m);
+        const int last = nz ? m * m : 0;
 #pragma unroll 1
-            for (int e = gl; e < m * m; e += G) {
+        for (int e0 = gl; e0 - gl < m * m; e0 += U * G) {
+            double aij[U], akj[U], aik[U];
+            int at[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int e = e0 + u * G;
                 const int ii = static_cast<int>((static_cast<unsigned>(e) * cm) >> 16);
                 const int i = k + 1 + ii;
                 const int j = k + 1 + (e - ii * m);
-                E[i * NEQ + j] = E[i * NEQ + j] + E[k * NEQ + j] * E[i * NEQ + k];
+                at[u] = i * NEQ + j;
+                if (e < last) {
+                    aij[u] = E[at[u]];
+                    akj[u] = E[k * NEQ + j];
+                    aik[u] = E[i * NEQ + k];
+                }
             }
-        } else {
-            info = k + 1;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (e0 + u * G < last) E[at[u]] = aij[u] + akj[u] * aik[u];
         }
-        __syncwarp(gmask);
+        __syncwarp();
     }
     piv |= static_cast<uint64_t>(NEQ - 1) << (4 * (NEQ - 1));
     if (E[(NEQ - 1) * NEQ + NEQ - 1] == 0.0) info = NEQ;
@@ -304,11 +390,11 @@ __device__ __forceinline__ int lu_coop(double* E, int gl, unsigned gmask, uint64
 // (c is uniform over the group; the register is picked by a select, so the
 // array stays in registers)
 template <int G, int K, class T>
-__device__ __forceinline__ T get(const T (&x)[K], int c, unsigned gmask) {
+__device__ __forceinline__ T get(const T (&x)[K], int c) {
     T v = x[0];
 #pragma unroll
     for (int t = 1; t < K; ++t) v = (c / G == t) ? x[t] : v;
-    return __shfl_sync(gmask, v, c % G, G);
+    return __shfl_sync(kWarp, v, c % G, G);
 }
 
 // the reciprocals of the factorisation's diagonal for the back substitutions
@@ -325,41 +411,82 @@ __device__ __forceinline__ void diag_recips(const double* LU, uint64_t (&rY)[K],
 
 // lu_solve<15> (reproducer.cpp:154-181) with x distributed over the group; the
 // back substitution's quotients use the pivots' precomputed reciprocals (the same
-// IEEE quotients as a division)
+// IEEE quotients as a division).  The next column's factors are loaded while a
+// column's chain (broadcast, quotient, multiply, add) runs.
+template <int K>
+struct Vec {
+    double v[K];
+};
 template <int G, int K>
-__device__ __forceinline__ void solve_coop(const double* LU, uint64_t ip, const uint64_t (&rY)[K], double (&x)[K],
-                                           int gl, unsigned gmask) {
+__device__ __noinline__ Vec<K> solve_copy(const double* LU, uint64_t ip, uint64_t r0, uint64_t r1, Vec<K> b, int gl) {
+    const uint64_t rY2[2] = {r0, r1};
+    uint64_t rY[K];
+#pragma unroll
+    for (int t = 0; t < K; ++t) rY[t] = rY2[t];
+    double(&x)[K] = b.v;
+    const double* row[K];
+#pragma unroll
+    for (int t = 0; t < K; ++t) row[t] = LU + (gl + t * G < NEQ ? gl + t * G : 0) * NEQ;
+    double l[K], ln[K];
+#pragma unroll
+    for (int t = 0; t < K; ++t) l[t] = row[t][0];
 #pragma unroll 1
     for (int k = 0; k < NEQ - 1; ++k) {
+#pragma unroll
+        for (int t = 0; t < K; ++t) ln[t] = row[t][k + 1];
         const int p = static_cast<int>((ip >> (4 * k)) & 15);
-        if (p != k) {
-            const double xk = get<G, K>(x, k, gmask);
-            const double xp = get<G, K>(x, p, gmask);
+        double tk = get<G, K>(x, k);
+        if (__any_sync(kWarp, p != k)) {
+            double v = x[0];
+#pragma unroll
+            for (int t = 1; t < K; ++t) v = (p / G == t) ? x[t] : v;
+            const double xp = __shfl_sync(kWarp, v, p % G, G);
 #pragma unroll
             for (int t = 0; t < K; ++t) {
                 const int c = gl + t * G;
-                x[t] = c == k ? xp : (c == p ? xk : x[t]);
+                x[t] = c == k ? xp : (c == p ? tk : x[t]);
             }
+            tk = xp;
         }
-        const double tk = get<G, K>(x, k, gmask);
 #pragma unroll
         for (int t = 0; t < K; ++t) {
             const int c = gl + t * G;
-            if (c > k && c < NEQ) x[t] = x[t] + tk * LU[c * NEQ + k];
+            if (c > k && c < NEQ) x[t] = x[t] + tk * l[t];
+            l[t] = ln[t];
         }
     }
+    // l holds column NEQ - 1
+    double d = LU[(NEQ - 1) * NEQ + NEQ - 1];
 #pragma unroll 1
     for (int k = NEQ - 1; k >= 0; --k) {
-        const uint64_t yk = get<G, K>(rY, k, gmask);
-        const double q = ddiv_recip(get<G, K>(x, k, gmask), LU[k * NEQ + k], yk);
+        const int kn = k > 0 ? k - 1 : 0;
+#pragma unroll
+        for (int t = 0; t < K; ++t) ln[t] = row[t][kn];
+        const double dn = LU[kn * NEQ + kn];
+        const uint64_t yk = get<G, K>(rY, k);
+        const double q = ddiv_recip(get<G, K>(x, k), d, yk);
         const double tk = -q;
 #pragma unroll
         for (int t = 0; t < K; ++t) {
             const int c = gl + t * G;
             if (c == k) x[t] = q;
-            if (c < k) x[t] = x[t] + tk * LU[c * NEQ + k];
+            if (c < k) x[t] = x[t] + tk * l[t];
+            l[t] = ln[t];
         }
+        d = dn;
     }
+    return b;
+}
+template <int G, int K>
+__device__ __forceinline__ void solve_coop(const double* LU, uint64_t ip, const uint64_t (&rY)[K], double (&x)[K],
+                                           int gl) {
+    static_assert(K <= 2, "15 unknowns on at least 8 lanes");
+    Vec<K> b;
+#pragma unroll
+    for (int t = 0; t < K; ++t) b.v[t] = x[t];
+    b = solve_copy<G, K>(LU, ip, rY[0], rY[K - 1], b, gl);
+#pragma unroll
+    for (int t = 0; t < K; ++t) x[t] = b.v[t];
 }
 
 template <int G, int K>
@@ -380,22 +507,57 @@ __device__ __forceinline__ void load_outputs(const uint64_t* V, const uint16_t* 
     }
 }
 
+// one evaluation of the network at v (kind 0: Jacobian and RHS, 1: RHS): the
+// program's index, whose output tables hold; regime is the group's guess, replaced by
+// the regime of the temperature found
+// (returned: the index in the low half, the regime in the high half)
+template <class M, int G, class Tab, int K>
+__device__ __noinline__ int evaluate_copy(int kind, Vec<K> b, int regime, int gl, uint64_t* V) {
+    double(&v)[K] = b.v;
+    int r = __shfl_sync(kWarp, regime, 0);
+    if (__any_sync(kWarp, regime != r)) r = __any_sync(kWarp, regime == 0) ? 0 : Tab::kRegimes - 1;
+#pragma unroll 1
+    while (true) {
+        store_inputs<G, K>(V, v, gl);
+        __syncwarp();
+        run_prog<M, G, Tab>(2 * r + kind, gl, V);
+        const uint64_t T = fetch(V, Tab::out(2 * r + kind)[NEQ]);
+        regime = regime_of<Tab>(T);
+        const bool fits = r == 0 || (T > Tab::regime(r, 0) && T <= Tab::regime(r, 1));
+        if (__all_sync(kWarp, fits)) break;
+        __syncwarp();  // every lane has read T
+        r = 0;
+    }
+    return (2 * r + kind) | regime << 16;
+}
+template <class M, int G, class Tab, int K>
+__device__ __forceinline__ int evaluate(int kind, const double (&v)[K], int& regime, int gl, uint64_t* V) {
+    Vec<K> b;
+#pragma unroll
+    for (int t = 0; t < K; ++t) b.v[t] = v[t];
+    const int w = evaluate_copy<M, G, Tab, K>(kind, b, regime, gl, V);
+    regime = w >> 16;
+    return w & 0xffff;
+}
+
 // E = -J into the matrix slots after the Jacobian program.  The program uses the
 // matrix slots as scratch and keeps its results (the Jacobian entries and the
 // RHS) above them; the generated table names, per matrix entry r * 15 + c, the
 // slot (a reserved one for a constant entry) that holds J(r, c) with the negation
 // as an operand modifier.
 template <int G>
-__device__ __forceinline__ void gather_matrix(uint64_t* V, const uint16_t* jac, int gl, unsigned gmask) {
-#pragma unroll 1
+__device__ __forceinline__ void gather_matrix(uint64_t* V, const uint16_t* jac, int gl) {
+#pragma unroll 5
     for (int i = gl; i < NEQ * NEQ; i += G) V[kE + i] = fetch(V, jac[i]);
-    __syncwarp(gmask);
+    __syncwarp();
 }
 
 // Generated tables of one G, supplied by the translation unit that includes the
 // generated header (one unit per G keeps the large initialisers apart).
-//   Tab::kNV, Tab::kNR, Tab::kNF, Tab::kJSteps, Tab::kRSteps and device accessors
-//   jprog(), jlit(), rprog(), rlit(), jout(), jac(), rout(), vconst(), vfun().
+//   Tab::kNV, Tab::kNR, Tab::kNF, Tab::kRegimes and device accessors vconst(),
+//   vfun(), prog(), lit(), ctl(i) (control bytes of four steps), first(w) and steps(w)
+//   of program w = 2 * regime + kind, out(w) (RHS operands, then T), jac(regime) and
+//   regime(k, 0 or 1) (the temperatures between which regime k holds).
 
 }  // namespace coop
 
@@ -458,14 +620,16 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
     const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (slot * G));
     uint64_t* V = sm + static_cast<size_t>((threadIdx.x >> 5) * SLOTS + slot) * Tab::kNV;
     double* E = reinterpret_cast<double*>(V + kE);
-    init_reserved<M, G, Tab>(V, gl, gmask);
+    init_reserved<M, G, Tab>(V, gl);
     const int n = s.n;
     const unsigned int queued = ctl->queued;
 
     PhaseClock<PH> pc;
     Lane L;
     int cell = -1, g = 0;
-    bool have = false;
+    bool have = false;     // the group holds a cell
+    bool drained = false;  // it has seen the queue's end
+    int regime = 0;        // the temperature regime of its last evaluation
     double y[K], f0[K], ak1[K], ak2[K], w[K];
 #pragma unroll
     for (int t = 0; t < K; ++t) y[t] = f0[t] = ak1[t] = ak2[t] = w[t] = 0.0;
@@ -474,15 +638,15 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
 #pragma unroll 1
     while (true) {
         // ---- bring the group's cell to "ready for an attempt" (per group)
-        bool exhausted = false;
 #pragma unroll 1
         while (true) {
             if (!have) {
+                if (drained) break;
                 unsigned int q = 0;
                 if (gl == 0) q = atomicAdd(&ctl->queue, 1u);
                 q = __shfl_sync(gmask, q, 0, G);
                 if (q >= queued) {
-                    exhausted = true;
+                    drained = true;
                     break;
                 }
                 cell = s.order[q];
@@ -509,6 +673,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
                 L.n_step = L.n_accept = L.n_reject = L.n_jac = L.n_decomp = 0;
                 L.fresh = true;
                 have = true;
+                regime = regime_of<Tab>(bits(s.T[cell]));
             }
             if (!L.fresh) break;
             // outer-loop checks, reproducer.cpp:7236-7255
@@ -548,17 +713,31 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
             }
             break;
         }
-        if (exhausted) break;
+        __syncwarp();
+        // the warp's groups run every attempt in step; a group without a cell
+        // follows one that has one (same state, same branches) and commits nothing
+        const unsigned holders = __ballot_sync(kWarp, have);
+        if (holders == 0) break;
+        {
+            const int from = (__ffs(holders) - 1) / G * G + gl;
+#pragma unroll
+            for (int t = 0; t < K; ++t) {
+                const double o = __shfl_sync(kWarp, y[t], from);
+                y[t] = have ? y[t] : o;
+            }
+            const double oh = __shfl_sync(kWarp, L.h, from);
+            L.h = have ? L.h : oh;
+            const int og = __shfl_sync(kWarp, regime, from);
+            regime = have ? regime : og;
+        }
         pc.mark(PH_QUEUE);
         pc.attempt();
 
         // ---- one ROS2S attempt, reproducer.cpp:7259-7345
-        store_inputs<G, K>(V, y, gl);
-        __syncwarp(gmask);
-        run_prog<M, G>(Tab::jprog(), Tab::jlit(), Tab::kJSteps, gl, V, gmask);
+        const int jw = evaluate<M, G, Tab, K>(0, y, regime, gl, V);
         pc.mark(PH_JPROG);
-        load_outputs<G, K>(V, Tab::jout(), f0, gl);
-        gather_matrix<G>(V, Tab::jac(), gl, gmask);
+        load_outputs<G, K>(V, Tab::out(jw), f0, gl);
+        gather_matrix<G>(V, Tab::jac(jw / 2), gl);
         if (L.fresh) L.n_jac += 1;
         L.fresh = false;
         const double h = L.h;
@@ -568,39 +747,15 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
             const int c = gl + t * G;
             if (c < NEQ) E[c * NEQ + c] = E[c * NEQ + c] + fac;
         }
-        __syncwarp(gmask);
+        __syncwarp();
         pc.mark(PH_MISC);
-        const int info = lu_coop<G>(E, gl, gmask, ip);
-        if (info != 0) {
-            L.nsing += 1;
-            if (L.nsing >= 5) {
-                if (gl == 0) {
-                    const uint64_t st[7] = {
-                        static_cast<uint64_t>(L.n_step), static_cast<uint64_t>(3 * L.n_step),
-                        static_cast<uint64_t>(L.n_jac), static_cast<uint64_t>(L.n_decomp),
-                        static_cast<uint64_t>(3 * L.n_step), static_cast<uint64_t>(L.n_accept),
-                        static_cast<uint64_t>(L.n_reject)};
-#pragma unroll
-                    for (int k = 0; k < 7; ++k) s.stats[k * n + cell] += st[k];
-                    s.cost[cell] = L.n_step;
-                    record_failure(ctl + g, WR_LU_DECOMPOSITION_ERROR);
-                }
-                have = false;
-            } else {
-                L.h = h * 0.5;
-                L.reject = true;
-                L.last = false;
-            }
-            __syncwarp(gmask);
-            continue;
-        }
-        L.n_decomp += 1;
+        const int info = lu_coop<G>(E, gl, ip);
         uint64_t rY[K];
         diag_recips<G, K>(E, rY, gl);
         pc.mark(PH_LU);
 #pragma unroll
         for (int t = 0; t < K; ++t) ak1[t] = f0[t];
-        solve_coop<G, K>(E, ip, rY, ak1, gl, gmask);
+        solve_coop<G, K>(E, ip, rY, ak1, gl);
         pc.mark(PH_SOLVE);
         // stage 2
         {
@@ -611,17 +766,15 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
                 yn[t] = y[t] + kA21 * ak1[t];
                 w[t] = c21h * ak1[t];
             }
-            store_inputs<G, K>(V, yn, gl);
-            __syncwarp(gmask);
             pc.mark(PH_MISC);
-            run_prog<M, G>(Tab::rprog(), Tab::rlit(), Tab::kRSteps, gl, V, gmask);
+            const int rw = evaluate<M, G, Tab, K>(1, yn, regime, gl, V);
             pc.mark(PH_RPROG);
             double dy[K];
-            load_outputs<G, K>(V, Tab::rout(), dy, gl);
+            load_outputs<G, K>(V, Tab::out(rw), dy, gl);
 #pragma unroll
             for (int t = 0; t < K; ++t) w[t] += dy[t];
             pc.mark(PH_MISC);
-            solve_coop<G, K>(E, ip, rY, w, gl, gmask);
+            solve_coop<G, K>(E, ip, rY, w, gl);
             pc.mark(PH_SOLVE);
 #pragma unroll
             for (int t = 0; t < K; ++t) ak2[t] = w[t];
@@ -634,18 +787,16 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
                 yn[t] = y[t] + kA31 * ak1[t] + kA32 * ak2[t];
                 w[t] = ddiv(kC31 * ak1[t] + kC32 * ak2[t], h);
             }
-            __syncwarp(gmask);  // every lane has read the stage-2 outputs
-            store_inputs<G, K>(V, yn, gl);
-            __syncwarp(gmask);
+            __syncwarp();  // every lane has read the stage-2 outputs
             pc.mark(PH_MISC);
-            run_prog<M, G>(Tab::rprog(), Tab::rlit(), Tab::kRSteps, gl, V, gmask);
+            const int rw = evaluate<M, G, Tab, K>(1, yn, regime, gl, V);
             pc.mark(PH_RPROG);
             double dy[K];
-            load_outputs<G, K>(V, Tab::rout(), dy, gl);
+            load_outputs<G, K>(V, Tab::out(rw), dy, gl);
 #pragma unroll
             for (int t = 0; t < K; ++t) w[t] += dy[t];
             pc.mark(PH_MISC);
-            solve_coop<G, K>(E, ip, rY, w, gl, gmask);
+            solve_coop<G, K>(E, ip, rY, w, gl);
             pc.mark(PH_SOLVE);
         }
         // w = k3: candidate and error estimate, reproducer.cpp:7299-7304
@@ -663,20 +814,31 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
             sq[t] = term * term;
         }
         // err = sum over components in index order (0.0 + sq[0] == sq[0]: a square)
-        double err = get<G, K>(sq, 0, gmask);
+        double err = get<G, K>(sq, 0);
 #pragma unroll
-        for (int c = 1; c < NEQ; ++c) err = err + get<G, K>(sq, c, gmask);
+        for (int c = 1; c < NEQ; ++c) err = err + get<G, K>(sq, c);
         err = ::sqrt(ddiv(err, 15.0));
-        L.n_step += 1;
         // step-size controller, reproducer.cpp:7308-7344
-        const double raw_fac = ddiv(M::cbrt(err), kSafe);
+        const double raw_fac = ddiv(StepMath<M>::cbrt(err), kSafe);
         const double fac_step = smax(1.0 / kFacMax, smin(1.0 / kFacMin, raw_fac));
         double hnew = ddiv(h, fac_step);
-        if (err <= 1.0) {
+        int code = 0;  // a failure that ends the cell's burn
+        if (info != 0) {  // singular: the attempt counts for nothing (reproducer.cpp:7268-7277)
+            L.nsing += 1;
+            if (L.nsing >= 5) {
+                code = WR_LU_DECOMPOSITION_ERROR;
+            } else {
+                L.h = h * 0.5;
+                L.reject = true;
+                L.last = false;
+            }
+        } else if (err <= 1.0) {
+            L.n_decomp += 1;
+            L.n_step += 1;
             L.n_accept += 1;
             if (L.n_accept > 1) {
                 const double facgus = smax(1.0 / kFacMax,
-                    smin(1.0 / kFacMin, ddiv(ddiv(L.hacc, h) * M::cbrt(ddiv(err * err, L.erracc)), kSafe)));
+                    smin(1.0 / kFacMin, ddiv(ddiv(L.hacc, h) * StepMath<M>::cbrt(ddiv(err * err, L.erracc)), kSafe)));
                 hnew = ddiv(h, smax(fac_step, facgus));
             }
             L.hacc = h;
@@ -691,29 +853,32 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
             L.h = hnew;
             L.fresh = true;
         } else {
+            L.n_decomp += 1;
+            L.n_step += 1;
             L.reject = true;
             L.last = false;
             L.h = hnew;
             if (L.n_accept >= 1) L.n_reject += 1;
-            if (hnew == 0.0) {
-                // the reject loop's only exit besides acceptance: a step size that
-                // has underflowed to zero ends the cell with the reference's
-                // DT_UNDERFLOW (reproducer.cpp:7240) instead of retrying forever
-                if (gl == 0) {
-                    const uint64_t st[7] = {
-                        static_cast<uint64_t>(L.n_step), static_cast<uint64_t>(3 * L.n_step),
-                        static_cast<uint64_t>(L.n_jac), static_cast<uint64_t>(L.n_decomp),
-                        static_cast<uint64_t>(3 * L.n_step), static_cast<uint64_t>(L.n_accept),
-                        static_cast<uint64_t>(L.n_reject)};
-#pragma unroll
-                    for (int k = 0; k < 7; ++k) s.stats[k * n + cell] += st[k];
-                    s.cost[cell] = L.n_step;
-                    record_failure(ctl + g, WR_DT_UNDERFLOW);
-                }
-                have = false;
-            }
+            // the reject loop's only exit besides acceptance: a step size that has
+            // underflowed to zero ends the cell with the reference's DT_UNDERFLOW
+            // (reproducer.cpp:7240) instead of retrying forever
+            if (hnew == 0.0) code = WR_DT_UNDERFLOW;
         }
-        __syncwarp(gmask);  // the next attempt overwrites V: every lane is done with it
+        if (have && code != 0) {
+            if (gl == 0) {
+                const uint64_t st[7] = {
+                    static_cast<uint64_t>(L.n_step), static_cast<uint64_t>(3 * L.n_step),
+                    static_cast<uint64_t>(L.n_jac), static_cast<uint64_t>(L.n_decomp),
+                    static_cast<uint64_t>(3 * L.n_step), static_cast<uint64_t>(L.n_accept),
+                    static_cast<uint64_t>(L.n_reject)};
+#pragma unroll
+                for (int k = 0; k < 7; ++k) s.stats[k * n + cell] += st[k];
+                s.cost[cell] = L.n_step;
+                record_failure(ctl + g, code);
+            }
+            have = false;
+        }
+        __syncwarp();  // the next attempt overwrites V: every lane is done with it
         pc.mark(PH_CTL);
     }
     pc.flush(phases, lane);
@@ -729,35 +894,34 @@ __global__ void k_diag_coop_network(int n, const double* __restrict__ y, double*
     constexpr int SLOTS = 32 / G;
     extern __shared__ uint64_t sm[];
     const int lane = threadIdx.x & 31, slot = lane / G, gl = lane % G;
-    const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (slot * G));
     const int warp = threadIdx.x >> 5;
-    const int cell = (blockIdx.x * (blockDim.x >> 5) + warp) * SLOTS + slot;
-    if (cell >= n) return;
+    // the warp's groups run in step: one past the end repeats the last case
+    const int cell = min((blockIdx.x * static_cast<int>(blockDim.x >> 5) + warp) * SLOTS + slot, n - 1);
     uint64_t* V = sm + static_cast<size_t>(warp * SLOTS + slot) * Tab::kNV;
     const double* E = reinterpret_cast<const double*>(V + kE);
-    init_reserved<M, G, Tab>(V, gl, gmask);
+    init_reserved<M, G, Tab>(V, gl);
     double yy[K], out[K];
 #pragma unroll
     for (int t = 0; t < K; ++t) {
         const int c = gl + t * G;
         yy[t] = c < NEQ ? y[static_cast<size_t>(cell) * NEQ + c] : 0.0;
     }
-    store_inputs<G, K>(V, yy, gl);
-    __syncwarp(gmask);
-    run_prog<M, G>(Tab::jprog(), Tab::jlit(), Tab::kJSteps, gl, V, gmask);
-    load_outputs<G, K>(V, Tab::jout(), out, gl);
-    gather_matrix<G>(V, Tab::jac(), gl, gmask);
+    // the first run finds the temperature's regime, so the two that count run its programs
+    int regime = 0;
+    evaluate<M, G, Tab, K>(1, yy, regime, gl, V);
+    __syncwarp();
+    const int jw = evaluate<M, G, Tab, K>(0, yy, regime, gl, V);
+    load_outputs<G, K>(V, Tab::out(jw), out, gl);
+    gather_matrix<G>(V, Tab::jac(jw / 2), gl);
     for (int i = gl; i < NEQ * NEQ; i += G) J[static_cast<size_t>(cell) * NEQ * NEQ + i] = -E[i];
 #pragma unroll
     for (int t = 0; t < K; ++t) {
         const int c = gl + t * G;
         if (c < NEQ) f[static_cast<size_t>(cell) * NEQ + c] = out[t];
     }
-    __syncwarp(gmask);
-    store_inputs<G, K>(V, yy, gl);
-    __syncwarp(gmask);
-    run_prog<M, G>(Tab::rprog(), Tab::rlit(), Tab::kRSteps, gl, V, gmask);
-    load_outputs<G, K>(V, Tab::rout(), out, gl);
+    __syncwarp();
+    const int rw = evaluate<M, G, Tab, K>(1, yy, regime, gl, V);
+    load_outputs<G, K>(V, Tab::out(rw), out, gl);
 #pragma unroll
     for (int t = 0; t < K; ++t) {
         const int c = gl + t * G;
@@ -773,27 +937,29 @@ __global__ void k_diag_coop_lu(int n, const double* __restrict__ A, const double
     constexpr int SLOTS = 32 / G;
     extern __shared__ uint64_t sm[];
     const int lane = threadIdx.x & 31, slot = lane / G, gl = lane % G;
-    const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (slot * G));
     const int warp = threadIdx.x >> 5;
-    const int cell = (blockIdx.x * (blockDim.x >> 5) + warp) * SLOTS + slot;
-    if (cell >= n) return;
+    // the warp's groups run in step: one past the end repeats the last case
+    const int cell = min((blockIdx.x * static_cast<int>(blockDim.x >> 5) + warp) * SLOTS + slot, n - 1);
     double* E = reinterpret_cast<double*>(sm) + static_cast<size_t>(warp * SLOTS + slot) * NEQ * NEQ;
     for (int i = gl; i < NEQ * NEQ; i += G) E[i] = A[static_cast<size_t>(cell) * NEQ * NEQ + i];
-    __syncwarp(gmask);
+    __syncwarp();
     uint64_t ip = 0;
-    const int inf = lu_coop<G>(E, gl, gmask, ip);
+    const int inf = lu_coop<G>(E, gl, ip);
     double v[K];
 #pragma unroll
     for (int t = 0; t < K; ++t) {
         const int c = gl + t * G;
         v[t] = c < NEQ ? b[static_cast<size_t>(cell) * NEQ + c] : 0.0;
     }
-    if (inf == 0) {
-        uint64_t rY[K];
-        diag_recips<G, K>(E, rY, gl);
-        solve_coop<G, K>(E, ip, rY, v, gl, gmask);
-    }
-    __syncwarp(gmask);
+    uint64_t rY[K];
+    diag_recips<G, K>(E, rY, gl);
+    double v2[K];
+#pragma unroll
+    for (int t = 0; t < K; ++t) v2[t] = v[t];
+    solve_coop<G, K>(E, ip, rY, v2, gl);
+#pragma unroll
+    for (int t = 0; t < K; ++t) v[t] = inf == 0 ? v2[t] : v[t];
+    __syncwarp();
     for (int i = gl; i < NEQ * NEQ; i += G) LU[static_cast<size_t>(cell) * NEQ * NEQ + i] = E[i];
 #pragma unroll
     for (int t = 0; t < K; ++t) {

@@ -26,7 +26,14 @@ constexpr int kPrepareThreads = 256;
 //   arrays fit in its shared memory, kWarps of generated/coop_prog_g<G>.h)
 constexpr int kAdvanceVariants = 8;
 constexpr int kPrecisionVariant = 3;
-constexpr int kDefaultVariant = 6;
+constexpr int kDefaultVariant = 6;   // 16 lanes per cell: the most cells per second
+constexpr int kLatencyVariant = 7;   // 32 lanes per cell: the shortest attempt
+// Cells per SM up to which a context takes 32 lanes per cell.  A block holds 16 cells
+// at 32 lanes and 32 at 16: while every cell has its warp at once, an outer step lasts
+// as long as its longest burn, and a 32-lane attempt is shorter (one outer step of 512
+// cells on GB300: 2.35 ms at 32 lanes, 3.24 ms at 16); beyond that the 16-lane shape's
+// rate decides (20,011 cells: 18.3 ms at 32 lanes, 13.3 ms at 16).
+constexpr int kLatencyCellsPerSm = 16;
 struct AdvanceShape {
     int threads;    // lane-per-cell shapes (0 for the cooperative advance)
     int blocks_per_sm;
@@ -37,6 +44,9 @@ struct AdvanceShape {
 constexpr AdvanceShape kAdvanceShapes[kAdvanceVariants] = {
     {128, 1, true, 0, 0},  {128, 2, false, 0, 0}, {256, 1, false, 0, 0},  {256, 1, true, 1, 0},
     {384, 1, false, 0, 0}, {0, 1, false, 0, 8}, {0, 1, false, 0, 16}, {0, 1, false, 0, 32}};
+constexpr int default_variant(int cells, int sms) {
+    return cells <= sms * kLatencyCellsPerSm ? kLatencyVariant : kDefaultVariant;
+}
 constexpr bool is_coop(int variant) { return kAdvanceShapes[variant].coop_lanes != 0; }
 
 constexpr size_t advance_smem_bytes(int variant) {

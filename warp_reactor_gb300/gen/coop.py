@@ -28,6 +28,11 @@ slot in the cell's own slot array, so the device adds it to one base):
 * literal word L: the lane's constant operand, XOR-ed into ``V[Y]`` (``Y`` then
   names a slot holding +0.0, so the operand is the constant); 0 otherwise.
 
+The device's tables hold the same steps with plain addresses in X, Y and Z, the class
+and the step flags in a control byte per step (``device_words``), and the device
+overlaps neighbouring steps: a main result is read at the earliest ``MAIN_DELAY``
+steps after its own.
+
 Constants therefore never need a table of their own: a network coefficient is the
 literal of the lane that uses it, and the few constants that integer nodes and the
 outputs read (booleans, the neutral operands 1, -1 and -0, comparison limits) sit
@@ -54,7 +59,9 @@ the separate operation:
 Comparisons are done on the bit patterns (exact IEEE ordering: NaN unordered,
 -0 == +0), booleans are stored as the integers 0/1, selects copy bit patterns.
 
-Two programs are generated per ``G``:
+Two programs are generated per ``G``, and for the wider lane counts (``REGIME_LANES``)
+the same two once more for each temperature range of ``REGIMES``, on which most of the
+network's piecewise conditions are known:
 
 * ``jrhs``: inputs ``y[0..14]`` (the ROS2S state: 14 number densities and the
   internal energy); prologue ``burn_state_from_y`` (reproducer.cpp:7029-7038):
@@ -87,9 +94,13 @@ the same operands wherever and whenever it is computed.
 from __future__ import annotations
 
 import collections
+import concurrent.futures
+import math
 import os
 import random
 import struct
+import subprocess
+import sys
 
 from . import ir_io
 
@@ -100,6 +111,7 @@ C_NONE, C_FMA, C_EXP, C_LOG, C_SQRT, C_DIV = 0, 1, 2, 3, 4, 5
 # operation on A (flip the sign bit, or clear it)
 I_SEL, I_LE, I_LT, I_SGN = 0, 1, 2, 3
 
+SPECIAL_OPS = ("le", "lt", "sneg", "sabs")  # integer nodes that are not selects
 FMA_OPS = ("add", "sub", "mul")
 MAIN_CLASS = {"add": C_FMA, "sub": C_FMA, "mul": C_FMA, "exp": C_EXP, "cexp": C_EXP, "log": C_LOG,
               "clog": C_LOG, "sqrt": C_SQRT, "csqrt": C_SQRT, "div": C_DIV}
@@ -127,6 +139,12 @@ FL_SABS = 4                              # D2 of I_SGN: clear the sign bit (else
 # so that the device may load four steps ahead without a bound check
 STEP_ALIGN = 4
 PREFETCH_PAD = 4
+# steps from a value's step to the first step that may read it: the device issues a
+# step's FP64 instruction, then stores the previous step's main results and loads the
+# next step's operands, so a main result is in shared memory two steps on, an integer
+# node's the next step
+MAIN_DELAY = 2
+INT_DELAY = 1
 SIGN = 1 << 63
 ABS = SIGN - 1
 # leaves of a program: inputs, constants, and transcendentals of constants
@@ -172,9 +190,10 @@ class Program:
         return self.const_bits(dbits(v))
 
 
-def build(dag, kind: str) -> tuple:
+def build(dag, kind: str, regime=None) -> tuple:
     """The program of ``kind`` ('jrhs' or 'rhs') and its outputs:
-    ``jac`` {(r, c): node} (jrhs only) and ``rhs`` [node] * 15."""
+    ``jac`` {(r, c): node} (jrhs only), ``rhs`` [node] * 15 and the temperature ``T``.
+    ``regime``: (lo, hi), the program for states with lo < T <= hi (``specialize``)."""
     P = Program()
     Y = [P.add("in", k) for k in range(15)]
     floor = P.const(FLOOR)
@@ -212,8 +231,87 @@ def build(dag, kind: str) -> tuple:
     out = {"rhs": [m[dag.outputs[("rhs", i)]] for i in range(15)]}
     if kind == "jrhs":
         out["jac"] = {(r, c): m[dag.outputs[("jac", r, c)]] for r in range(15) for c in range(15)}
+    out["T"] = T
+    if regime is not None:
+        P, out = specialize(P, out, *regime)
     rebalance_boolean_chains(P)
     return P, out
+
+
+def specialize(P: Program, out: dict, lo: float, hi: float) -> tuple:
+    """The program for states with lo < T <= hi.  A comparison of T, or of T times or
+    plus constants (monotone in T also in binary64), with a constant is decided where
+    both ends of the interval decide it alike; boolean logic and selects on decided
+    conditions reduce to the operand they would choose, so every value that remains is
+    the same operation on the same operands as in the general program."""
+    T = out["T"]
+
+    def const(x):
+        b, neg, ab = resolve(P, x)
+        if P.nodes[b][0] != "const":
+            return None
+        v = struct.unpack("<d", struct.pack("<Q", P.nodes[b][1][0]))[0]
+        v = abs(v) if ab else v
+        return -v if neg else v
+
+    ends = {T: (math.nextafter(lo, math.inf), hi)}
+
+    def interval(x):
+        if x not in ends:
+            op, a = P.nodes[x]
+            r = None
+            if op in FMA_OPS:
+                k = [const(y) for y in a]
+                if k[0] is None and k[1] is not None and interval(a[0]):
+                    fn = {"mul": lambda v: v * k[1], "add": lambda v: v + k[1], "sub": lambda v: v - k[1]}[op]
+                    r = sorted(map(fn, interval(a[0])))
+                elif k[1] is None and k[0] is not None and interval(a[1]):
+                    fn = {"mul": lambda v: v * k[0], "add": lambda v: v + k[0], "sub": lambda v: k[0] - v}[op]
+                    r = sorted(map(fn, interval(a[1])))
+            elif op == "const":
+                r = (const(x), const(x))
+            ends[x] = r
+        return ends[x]
+
+    Q = Program()
+    false, true = Q.const_bits(0), Q.const_bits(1)
+    memo, m = {}, {}
+
+    def node(op, *args):
+        key = (op,) + args
+        if key not in memo:
+            memo[key] = Q.add(op, *args)
+        return memo[key]
+
+    for x, (op, a) in enumerate(P.nodes):  # operands come before their users
+        r = None
+        if op == "const":
+            m[x] = Q.const_bits(a[0])
+            continue
+        if op == "in":
+            m[x] = node(op, *a)
+            continue
+        b = [m[y] for y in a]
+        if op in ("le", "lt"):
+            i, j = interval(a[0]), interval(a[1])
+            if i and j:
+                if (i[1] <= j[0]) if op == "le" else (i[1] < j[0]):
+                    r = true
+                elif (i[0] > j[1]) if op == "le" else (i[0] >= j[1]):
+                    r = false
+        elif op == "and":
+            r = false if false in b else b[1] if b[0] == true else b[0] if b[1] == true or b[0] == b[1] else None
+        elif op == "or":
+            r = true if true in b else b[1] if b[0] == false else b[0] if b[1] == false or b[0] == b[1] else None
+        elif op == "not":
+            r = false if b[0] == true else true if b[0] == false else None
+        elif op == "sel":
+            r = b[1] if b[0] == true or b[1] == b[2] else b[2] if b[0] == false else None
+        m[x] = node(op, *b) if r is None else r
+    new = {"rhs": [m[x] for x in out["rhs"]], "T": m[T]}
+    if "jac" in out:
+        new["jac"] = {k: m[x] for k, x in out["jac"].items()}
+    return Q, new
 
 
 BOOL_OPS = ("and", "or", "not")
@@ -370,7 +468,7 @@ def live_nodes(P: Program, roots, leaves=False) -> list:
 
 
 def roots_of(out: dict) -> list:
-    return list(out["rhs"]) + ([x for _, x in sorted(out["jac"].items())] if "jac" in out else [])
+    return list(out["rhs"]) + [out["T"]] + ([x for _, x in sorted(out["jac"].items())] if "jac" in out else [])
 
 
 def device_constants(P: Program, out: dict) -> set:
@@ -406,15 +504,20 @@ class Schedule:
         self.consts = consts
 
 
-def list_schedule(comp, args, users, kind, prio, G, limit=None, hold=None):
+def list_schedule(comp, args, users, kind, prio, G, limit=None, hold=None, fill=0):
     """Steps of width G: each step takes up to G ready nodes of one main class
     (highest priority first; a full step is preferred) and up to G ready integer
-    nodes.  ``args``/``users`` give the dependences in the direction scheduled.
+    nodes.  ``args``/``users`` give the dependences in the direction scheduled.  A
+    node is ready ``MAIN_DELAY`` steps after its last main operand (``INT_DELAY``
+    after an integer one); a step with nothing ready stays empty.
 
     ``hold``: a partial exp/log/sqrt step costs as many FP64 issue slots as a full
     one, so while an FMA or division step can be filled instead, a transcendental
     class is taken only if its most critical ready node leads theirs by more than
     ``hold`` (a number, or one per class; None: no such rule).
+
+    ``fill``: with fewer ready FMA nodes than that, and more becoming ready at the next
+    step, a step is left without a main node (never two in a row).
 
     ``limit``: once that many computed values are live (computed, with users not
     yet scheduled), ready nodes are taken by their effect on the live set first
@@ -426,6 +529,8 @@ def list_schedule(comp, args, users, kind, prio, G, limit=None, hold=None):
     for x in comp:
         if pend[x] == 0:
             ready[kind(x)].append(x)
+    earliest = collections.defaultdict(int)   # first step that may read all of a node's operands
+    later = collections.defaultdict(list)     # nodes that become ready at a later step
     steps = []
     left = len(comp)
     live = 0
@@ -441,11 +546,17 @@ def list_schedule(comp, args, users, kind, prio, G, limit=None, hold=None):
         return max(prio[x] for x in ready[c])
 
     while left:
+        for x in later.pop(len(steps), []):
+            ready[kind(x)].append(x)
         rl = sorted(ready["int"], key=key)
         riders, ready["int"] = rl[:G], rl[G:]
         cand = [c for c in mains if ready[c]]
         cls, take = C_NONE, []
-        if cand:
+        # a thin step now and the rest of its nodes one step later would take two FP64
+        # issue slots: wait for them
+        wait = (cand and later.get(len(steps) + 1) and len(ready[C_FMA]) < fill and
+                all(len(ready[c]) < G for c in cand) and not (steps and steps[-1][0] == C_NONE))
+        if cand and not wait:
             full = [c for c in cand if len(ready[c]) >= G]
             pool = full if full else cand
             cheap = [c for c in cand if c in (C_FMA, C_DIV)]
@@ -456,6 +567,7 @@ def list_schedule(comp, args, users, kind, prio, G, limit=None, hold=None):
             cls = max(pool, key=lambda c: (top(c), len(ready[c])))
             rl = sorted(ready[cls], key=key)
             take, ready[cls] = rl[:G], rl[G:]
+        s = len(steps)
         steps.append((cls, take, riders))
         left -= len(take) + len(riders)
         for x in take + riders:
@@ -464,17 +576,22 @@ def list_schedule(comp, args, users, kind, prio, G, limit=None, hold=None):
                 remaining[a] -= 1
                 live -= 1 if remaining[a] == 0 else 0
             for u in users[x]:
+                earliest[u] = max(earliest[u], s + delay(kind(x)))
                 pend[u] -= 1
                 if pend[u] == 0:
-                    ready[kind(u)].append(u)
+                    later[earliest[u]].append(u)
     return steps
+
+
+def delay(kind) -> int:
+    return INT_DELAY if kind == "int" else MAIN_DELAY
 
 
 def sink_riders(steps, users, kind, G):
     """Move every integer node with users to the latest step before its first
     user that has a free integer lane (integer nodes cost no FP64 issue slot, so
-    computing them late only shortens their values' lives); steps left empty are
-    dropped."""
+    computing them late only shortens their values' lives).  Steps stay where they
+    are: an empty one keeps its users' distance from the step before it."""
     done = {}
     for s, (_, take, riders) in enumerate(steps):
         for x in take + riders:
@@ -488,7 +605,7 @@ def sink_riders(steps, users, kind, G):
                 lanes[s].append(x)
                 done[x] = s
                 break
-    return [(cls, take, lanes[s]) for s, (cls, take, _) in enumerate(steps) if take or lanes[s]]
+    return [(cls, take, lanes[s]) for s, (cls, take, _) in enumerate(steps)]
 
 
 def schedule(P: Program, out: dict, G: int, jac: bool, limit=None, first_scratch=RES_BASE, tune=None,
@@ -504,13 +621,13 @@ def schedule(P: Program, out: dict, G: int, jac: bool, limit=None, first_scratch
     ``first_scratch``: the first slot above the reserved constants.  ``tune``:
     (latency weight of exp/log/sqrt, ``hold`` of the list scheduler, seed of a
     random perturbation of the priorities (0: none)[, its amplitude, 1e-3 by
-    default]) -- the schedule is a heuristic, and these pick among equally valid
+    default[, ``fill`` of the list scheduler]]) -- the schedule is a heuristic, and these pick among equally valid
     ones.  ``banked``: (reserved slot map, slot cap) to allocate slots with
     ``allocate_banked`` (G = 16), falling back to the linear scan when it finds
     no room below the cap."""
     leaf = LEAF
     jac_roots = [x for _, x in sorted(out["jac"].items())] if jac else []
-    roots = list(out["rhs"]) + jac_roots
+    roots = list(out["rhs"]) + [out["T"]] + jac_roots
     comp = live_nodes(P, roots)
     args = {x: [resolve(P, a)[0] for a in P.nodes[x][1]] for x in comp}
     cargs = {x: sorted({a for a in args[x] if P.nodes[a][0] not in leaf}) for x in comp}
@@ -531,21 +648,21 @@ def schedule(P: Program, out: dict, G: int, jac: bool, limit=None, first_scratch
             if pend[u] == 0:
                 order.append(u)
     assert len(order) == len(comp), "the program has a cycle"
-    lat_t, hold, seed, amp = (tuple(tune) + (1e-3,))[:4] if tune else (LATENCY[C_EXP], None, 0, 0.0)
+    lat_t, hold, seed, amp, fill = (tuple(tune) + (1e-3, 0)[len(tune) - 3:])[:5] if tune else (LATENCY[C_EXP], None, 0, 0.0, 0)
     lat = dict(LATENCY)
-    lat.update({C_EXP: lat_t, C_LOG: lat_t, C_SQRT: max(1.0, lat_t - 1.0)})
+    lat.update({C_FMA: float(MAIN_DELAY), C_DIV: 3.0, C_EXP: lat_t, C_LOG: lat_t, C_SQRT: max(1.0, lat_t - 1.0)})
     rng = random.Random(seed)
     prio = {}
     for x in reversed(order):
         prio[x] = lat[kind(x)] + max((prio[u] for u in users[x]), default=0.0)
         prio[x] += rng.random() * amp if seed else 0.0
-    steps = sink_riders(list_schedule(comp, cargs, users, kind, prio, G, limit, hold), users, kind, G)
+    steps = sink_riders(list_schedule(comp, cargs, users, kind, prio, G, limit, hold, fill), users, kind, G)
     done_at = {}
     for s, (cls, take, riders) in enumerate(steps):
         for x in take + riders:
             done_at[x] = s
     for x in comp:
-        assert all(done_at[a] < done_at[x] for a in cargs[x]), "schedule violates a dependence"
+        assert all(done_at[a] + delay(kind(a)) <= done_at[x] for a in cargs[x]), "schedule violates a dependence"
     # ---- slot allocation (linear scan; a slot read last in step s is free from
     # s+1).  Two pools: the matrix slots (scratch of the Jacobian program only)
     # and the slots above the inputs; kept values come from the upper pool.
@@ -562,7 +679,7 @@ def schedule(P: Program, out: dict, G: int, jac: bool, limit=None, first_scratch
         got = allocate_banked(P, steps, last, keep, inputs, banked[0], jac, first_scratch, banked[1] - 1)
         if got is not None:
             slot, nv = got
-            outputs = {"rhs": [resolve(P, r) for r in out["rhs"]]}
+            outputs = {"rhs": [resolve(P, r) for r in out["rhs"]], "T": resolve(P, out["T"])}
             if jac:
                 outputs["jac"] = [resolve(P, x) for x in jac_roots]
             return Schedule(G, steps, slot, nv + 1, outputs, None), args  # + the write sink
@@ -598,7 +715,7 @@ def schedule(P: Program, out: dict, G: int, jac: bool, limit=None, first_scratch
     nv += 1  # write sink of idle lanes
     if nv > MAX_SLOTS:
         raise ValueError(f"program needs {nv} slots (max {MAX_SLOTS})")
-    outputs = {"rhs": [resolve(P, r) for r in out["rhs"]]}
+    outputs = {"rhs": [resolve(P, r) for r in out["rhs"]], "T": resolve(P, out["T"])}
     if jac:
         outputs["jac"] = [resolve(P, x) for x in jac_roots]
     return Schedule(G, steps, slot, nv, outputs, None), args
@@ -852,7 +969,7 @@ def encode(P: Program, sch: Schedule, res: dict) -> list:
 
     words = []
     for cls, take, riders in sch.steps:
-        special = any(P.nodes[x][0] in ("le", "lt", "sneg", "sabs") for x in riders)
+        special = any(P.nodes[x][0] in SPECIAL_OPS for x in riders)
         zfl = (FL_INT if riders else 0) | (FL_SPECIAL if special else 0)
         lanes = []
         for g in range(G):
@@ -925,16 +1042,94 @@ def encode(P: Program, sch: Schedule, res: dict) -> list:
     return words + [idle] * PREFETCH_PAD
 
 
+# device words (device_words): flags in the low bits of D
+DV_NEG, DV_ABS, DV_SWAP = 1, 2, 4        # exp/log/sqrt: on V[Y] ^ L (abs, then negate); division: on V[X]
+# control byte: class | integer nodes | comparisons or sign operations among them |
+# store the main results in the step itself
+CTL_INT, CTL_SPECIAL, CTL_FLUSH = 8, 16, 32
+DEVICE_ALIGN = 4                         # steps per iteration of the device's loop
+
+
+def device_words(pr: dict, nv: int) -> tuple:
+    """The words of an encoded program as the device executes them, and one control
+    byte per step.  The device loads every step's X, Y and Z before it looks at the
+    step's class, so these fields carry plain addresses: the class and the step flags
+    move to the control byte, the sign modifiers to the low bits of D (a negation of
+    V[Y] without an absolute value is a sign flip of the literal).  A step that only
+    keeps its neighbours apart disappears: the step before it stores its main results
+    itself (``CTL_FLUSH``), so the step after may read them.  Idle steps, which store
+    into the write sink, pad the program to ``DEVICE_ALIGN``, then ``PREFETCH_PAD``."""
+    sink = ((nv - 1) << 3) << 48
+    words, ctl = [], []
+    for lanes in pr["words"][:pr["nsteps"]]:
+        m0 = lanes[0][0]
+        cls, zfl = (m0 >> 48) & 7, (m0 >> 32) & 7
+        if cls == C_NONE and not zfl & FL_INT:
+            if ctl:
+                ctl[-1] |= CTL_FLUSH if ctl[-1] & 7 else 0
+            continue
+        ctl.append(cls | (CTL_INT if zfl & FL_INT else 0) | (CTL_SPECIAL if zfl & FL_SPECIAL else 0))
+        out = []
+        for m, i, lit in lanes:
+            x, y, z, d = ((m >> (16 * k)) & 0xffff for k in range(4))
+            xf, yf, fl = x & 7, y & 7, 0
+            if cls == C_NONE:
+                d = sink >> 48
+            elif cls == C_DIV:
+                assert not yf & FL_ABS, "absolute value on the literal side of a division"
+                fl = (DV_NEG if xf & FL_NEG else 0) | (DV_ABS if xf & FL_ABS else 0) | (DV_SWAP if yf & FL_SWAP else 0)
+                lit ^= SIGN if yf & FL_NEG else 0
+            elif cls != C_FMA:
+                if yf & FL_ABS:
+                    fl = DV_ABS | (DV_NEG if yf & FL_NEG else 0)
+                else:
+                    lit ^= SIGN if yf & FL_NEG else 0
+            out.append(((x & ~7) | ((y & ~7) << 16) | ((z & ~7) << 32) | (((d & ~7) | fl) << 48), i, lit))
+        words.append(out)
+    pad = -len(words) % DEVICE_ALIGN + PREFETCH_PAD
+    return words + [[(sink, 0, 0)] * len(lanes)] * pad, ctl + [C_NONE] * pad
+
+
 # live-set limit of the list scheduler per G (chosen offline: the smallest slot
 # count among limits that do not add FP64 issue slots)
-SCHED_LIMIT = {8: 400, 16: 650, 32: None}
+SCHED_LIMIT = {8: 400, 16: 350, 32: 600}
 # scheduler tuning per G and program: (schedule()'s ``tune``, live-set limit),
 # chosen offline by a seeded random search for the fewest FP64 issue slots of the
 # program whose slot count keeps the block's warps (16 lanes: 16 warps, <= 907
 # slots; 8 lanes: 9 warps, <= 807 slots)
 SCHED_TUNE = {
-    16: {"jrhs": ((6.0, 3.0, 588627), 550), "rhs": ((1.5, None, 405133), 550)},
-    8: {"jrhs": ((2.0, 0.0, 509381), 400), "rhs": ((2.0, 1.0, 795782), 500)},
+    16: {
+        "jrhs": ((2.0, 8.0, 80444, 0.01, 8), 350),
+        "rhs": ((4.0, 8.0, 913542, 0.5, 14), 425),
+        (1, "jrhs"): ((3.0, None, 998460, 0.01, 14), 350),
+        (1, "rhs"): ((1.5, {C_EXP: 2.0, C_LOG: 2.0, C_SQRT: 20.0}, 109686, 1.0, 14), 600),
+        (2, "jrhs"): ((4.0, 0.0, 68050, 1.0, 11), 500),
+        (2, "rhs"): ((4.5, 8.0, 105236, 0.001, 13), 600),
+        (3, "jrhs"): ((2.0, 1.0, 544639, 0.001, 11), 450),
+        (3, "rhs"): ((3.0, {C_EXP: 0.0, C_LOG: 10.0, C_SQRT: 20.0}, 505950, 0.5, 13), 475),
+        (4, "jrhs"): ((3.0, 0.0, 164671, 0.001, 10), 600),
+        (4, "rhs"): ((1.0, 8.0, 634925, 0.01, 11), 650),
+        (5, "jrhs"): ((6.5, 1.0, 275871, 0.5, 11), 600),
+        (5, "rhs"): ((2.0, {C_EXP: 2.0, C_LOG: 10.0, C_SQRT: 20.0}, 11048, 0.5, 13), 550),
+        (6, "jrhs"): ((8.0, None, 437426, 0.001, 10), 475),
+        (6, "rhs"): ((3.5, {C_EXP: 2.0, C_LOG: 30.0, C_SQRT: 5.0}, 6388, 0.5, 12), 450),
+    },
+    32: {
+        "jrhs": ((1.5, 0.0, 849342, 0.001, 20), 600),
+        "rhs": ((8.0, {C_EXP: 20.0, C_LOG: 30.0, C_SQRT: 5.0}, 620078, 0.1, 23), 450),
+        (1, "jrhs"): ((5.5, None, 378914, 0.1, 30), 525),
+        (1, "rhs"): ((3.5, {C_EXP: 20.0, C_LOG: 30.0, C_SQRT: 5.0}, 499564, 2.0, 21), 600),
+        (2, "jrhs"): ((2.5, 0.0, 16209, 0.001, 19), 600),
+        (2, "rhs"): ((1.5, 8.0, 723724, 2.0, 23), 550),
+        (3, "jrhs"): ((5.5, 2.0, 789616, 0.5, 30), 500),
+        (3, "rhs"): ((4.5, {C_EXP: 20.0, C_LOG: 10.0, C_SQRT: 20.0}, 602532, 2.0, 10), 600),
+        (4, "jrhs"): ((6.0, 5.0, 173831, 0.5, 31), 375),
+        (4, "rhs"): ((1.0, {C_EXP: 20.0, C_LOG: 5.0, C_SQRT: 0.0}, 421877, 1.0, 32), 700),
+        (5, "jrhs"): ((4.0, 0.0, 585544, 0.001, 19), 600),
+        (5, "rhs"): ((8.0, {C_EXP: 20.0, C_LOG: 30.0, C_SQRT: 5.0}, 845573, 2.0, 24), 450),
+        (6, "rhs"): ((7.0, {C_EXP: 20.0, C_LOG: 30.0, C_SQRT: 5.0}, 391120, 1.0, 31), 450),
+    },
+    8: {"jrhs": ((1.5, 8.0, 899089, 0.5, 7), 400), "rhs": ((1.5, 8.0, 27320, 1.0, 2), 650)},
 }
 # shared memory of one block (227 KiB) and the warps per block the slot arrays
 # allow, at most 16: at 16 lanes per cell (728 slots) 16 warps ran a 64^3 collapse
@@ -953,11 +1148,24 @@ def warps_per_block(G: int, nv: int) -> int:
     return max(1, min(MAX_WARPS, cells // (32 // G)))
 
 
-def generate(G: int, dag=None, limit="default", tune="default", banked="default"):
+# Temperature regimes with programs of their own (lo < T <= hi): the network's fits
+# change at 200, 500, 1000, 1160, 1167.48, 2000 and 6000 K, and between two of them a
+# program has 10 % fewer adds and multiplies, 12 % fewer exponentials and 80 % fewer
+# integer nodes than the general one.  The last one spans them all (4 % fewer, 45 %
+# fewer integer nodes), for a warp whose cells lie in different regimes.
+REGIMES = ((200.0, 500.0), (500.0, 1000.0), (1000.0, 1160.0), (1167.479642374226, math.nextafter(2000.0, 0.0)),
+           (math.nextafter(2000.0, 0.0), 6000.0), (200.0, 6000.0))
+# lane widths whose kernels carry the regimes' programs
+REGIME_LANES = (16, 32)
+
+
+def generate(G: int, dag=None, limit="default", tune="default", banked="default", regimes=()):
     """Programs jrhs and rhs for G lanes per cell: a dict with the encoded steps,
     the output operands, the slot count, the reserved constants and the warps
     per block.  ``banked``: allocate slots with ``allocate_banked`` within the
-    slot count that keeps the block's warps (G = 16)."""
+    slot count that keeps the block's warps (G = 16).  ``regimes``: also the programs
+    of these temperature regimes (``regimes``: a list of {lo, hi, progs}), on the same
+    slot map and reserved constants."""
     dag = dag or ir_io.load()
     if limit == "default":
         limit = SCHED_LIMIT.get(G)
@@ -966,12 +1174,13 @@ def generate(G: int, dag=None, limit="default", tune="default", banked="default"
     built = {}
     pool = {0, 1, dbits(1.0), dbits(-1.0), dbits(-0.0)}
     funs = set()
-    for kind in ("jrhs", "rhs"):
-        P, out = build(dag, kind)
-        lower(P)
-        pool |= reserved_constants(P, out)
-        funs |= device_constants(P, out)
-        built[kind] = (P, out)
+    for reg in (None,) + tuple(regimes):
+        for kind in ("jrhs", "rhs"):
+            P, out = build(dag, kind, reg)
+            lower(P)
+            pool |= reserved_constants(P, out)
+            funs |= device_constants(P, out)
+            built[reg, kind] = (P, out)
     # reserved slots: false/+0.0, true, 1, -1, -0 first, then the rest in order,
     # then the transcendentals of constants
     fixed = [0, 1, dbits(1.0), dbits(-1.0), dbits(-0.0)]
@@ -986,18 +1195,19 @@ def generate(G: int, dag=None, limit="default", tune="default", banked="default"
     # block's whole shared memory
     cap = max(nv for nv in range(first, MAX_SLOTS) if warps_per_block(G, nv) == MAX_WARPS) - 1
     scheds = {}
-    for kind, (P, out) in built.items():
-        t, lim = (tune or {}).get(kind, (None, limit))
-        scheds[kind] = schedule(P, out, G, jac=(kind == "jrhs"), limit=lim, first_scratch=first, tune=t,
-                                banked=(res, cap) if banked else None)
+    for (reg, kind), (P, out) in built.items():
+        key = kind if reg is None else (REGIMES.index(reg) + 1, kind)
+        t, lim = (tune or {}).get(key, (tune or {}).get(kind, (None, limit)))
+        scheds[reg, kind] = schedule(P, out, G, jac=(kind == "jrhs"), limit=lim, first_scratch=first, tune=t,
+                                     banked=(res, cap) if banked else None)
     nv = max(sch.nv for sch, _ in scheds.values())
     if nv * 8 > 0xfff8:
         raise ValueError(f"{nv} slots do not fit the 16-bit byte offsets")
     progs = {}
-    for kind, (P, out) in built.items():
-        sch, _ = scheds[kind]
+    for (reg, kind), (P, out) in built.items():
+        sch, _ = scheds[reg, kind]
         st = stats(sch)
-        sch.nv = nv  # one slot map (and one write sink, the last slot) for both programs
+        sch.nv = nv  # one slot map (and one write sink, the last slot) for all programs
         words = encode(P, sch, res)
 
         def outop(r, negate=False):
@@ -1008,11 +1218,13 @@ def generate(G: int, dag=None, limit="default", tune="default", banked="default"
             v = res[P.nodes[b][1][0]] if op == "const" else res[P.nodes[b][1]] if op == "dconst" else sch.slot[b]
             return v | (OPF_NEG if neg else 0) | (OPF_ABS if ab else 0)
 
-        progs[kind] = {"words": words, "rhs_out": [outop(r) for r in sch.outputs["rhs"]],
-                       "nsteps": len(words) - PREFETCH_PAD, "stats": st}
+        pr = {"words": words, "rhs_out": [outop(r) for r in sch.outputs["rhs"]], "T_out": outop(sch.outputs["T"]),
+              "nsteps": len(words) - PREFETCH_PAD, "stats": st}
         if "jac" in sch.outputs:  # E = -J, entry r * 15 + c
-            progs[kind]["jac_out"] = [outop(r, negate=True) for r in sch.outputs["jac"]]
-    return {"G": G, "nv": nv, "rconst": rconst, "rfun": rfun, "progs": progs, "warps": warps_per_block(G, nv)}
+            pr["jac_out"] = [outop(r, negate=True) for r in sch.outputs["jac"]]
+        progs.setdefault(reg, {})[kind] = pr
+    return {"G": G, "nv": nv, "rconst": rconst, "rfun": rfun, "progs": progs[None], "warps": warps_per_block(G, nv),
+            "regimes": [{"lo": r[0], "hi": r[1], "progs": progs[r]} for r in regimes]}
 
 
 def shared_wavefronts(pr: dict) -> dict:
@@ -1071,10 +1283,27 @@ def emit_header(G: int, gen: dict, digest: str) -> str:
         f"constexpr int kNF = {len(gen['rfun'])};  // then the transcendentals of constants",
         f"constexpr int kWarps = {gen['warps']};  // warps per block: the slot arrays that fit in shared memory",
     ]
-    for kind, pr in gen["progs"].items():
+    # every program in one table: the general ones first, then each regime's
+    progs = [("general", p) for p in gen["progs"].items()]
+    for r in gen["regimes"]:
+        progs += [(f"{r['lo']:g} < T <= {r['hi']:g}", p) for p in r["progs"].items()]
+    nreg = 1 + len(gen["regimes"])
+    lines.append(f"constexpr int kRegimes = {nreg};  // 0: any state, the others by temperature")
+    lines.append("// first step and steps of each program: Jacobian + RHS and RHS of regime 0, 1, ...")
+    lines.append(f"static __constant__ const int kProgStep[{2 * nreg}][2] = {{")
+    dev = [device_words(pr, gen["nv"]) for _, (_, pr) in progs]
+    total = 0
+    for (what, (kind, pr)), (words, _) in zip(progs, dev):
         st = pr["stats"]
-        lines.append(f"constexpr int k{kind.upper()}Steps = {pr['nsteps']};  // {st['by_class']}, "
-                     f"{st['fp64_slots']:.0f} FP64 issue slots, {st['steps']} steps before padding")
+        lines.append(f"    {{{total}, {len(words) - PREFETCH_PAD}}},  // {kind}, {what}: {st['by_class']}, "
+                     f"{st['fp64_slots']:.0f} FP64 issue slots")
+        total += len(words)
+    lines.append("};")
+    lines.append("// lo < T <= hi as bit patterns (positive doubles order as integers)")
+    lines.append(f"static __constant__ const uint64_t kRegimeT[{nreg}][2] = {{{{0ULL, 0x7ff0000000000000ULL}},")
+    for r in gen["regimes"]:
+        lines.append(f"    {{0x{dbits(r['lo']):016x}ULL, 0x{dbits(r['hi']):016x}ULL}},")
+    lines.append("};")
     lines.append("")
     lines.append("static __device__ const uint64_t kVConst[kNR] = {")
     cs = gen["rconst"]
@@ -1086,25 +1315,32 @@ def emit_header(G: int, gen: dict, digest: str) -> str:
     for c, b in gen["rfun"] or [(0, 0)]:
         lines.append(f"    {{{c}ULL, 0x{b:016x}ULL}},")
     lines.append("};")
-    for kind, pr in gen["progs"].items():
-        K = kind.upper()
-        n = f"(k{K}Steps + {PREFETCH_PAD}) * kG"
-        lines.append(f"static __device__ const ulonglong2 k{K}Prog[{n}] = {{")
-        for lanes in pr["words"]:
+    lines.append("// control bytes, four steps to a word")
+    ctl = [sum(c[s + k] << (8 * k) for k in range(4)) for _, c in dev for s in range(0, len(c), 4)]
+    lines.append(f"static __constant__ const uint32_t kCtl[{len(ctl)}] = {{")
+    for i in range(0, len(ctl), 8):
+        lines.append("    " + ", ".join(f"0x{w:x}U" for w in ctl[i:i + 8]) + ",")
+    lines.append("};")
+    lines.append(f"static __device__ const ulonglong2 kProg[{total} * kG] = {{")
+    for words, _ in dev:
+        for lanes in words:
             lines.append("    " + ", ".join(f"{{0x{m:x}ULL, 0x{i:x}ULL}}" for m, i, _ in lanes) + ",")
-        lines.append("};")
-        lines.append(f"static __device__ const uint64_t k{K}Lit[{n}] = {{")
-        for lanes in pr["words"]:
+    lines.append("};")
+    lines.append(f"static __device__ const uint64_t kLit[{total} * kG] = {{")
+    for words, _ in dev:
+        for lanes in words:
             lines.append("    " + ", ".join(f"0x{l:x}ULL" for _, _, l in lanes) + ",")
-        lines.append("};")
-        lines.append(f"static __device__ const uint16_t k{K}Out[15] = {{" +
-                     ", ".join(str(v) for v in pr["rhs_out"]) + "};")
-        if "jac_out" in pr:
-            lines.append(f"static __device__ const uint16_t k{K}Jac[225] = {{")
-            jo = pr["jac_out"]
-            for i in range(0, 225, 15):
-                lines.append("    " + ", ".join(str(v) for v in jo[i:i + 15]) + ",")
-            lines.append("};")
+    lines.append("};")
+    lines.append("// output operands of each program: the RHS, then T")
+    lines.append(f"static __device__ const uint16_t kOut[{2 * nreg}][16] = {{")
+    for _, (_, pr) in progs:
+        lines.append("    {" + ", ".join(str(v) for v in pr["rhs_out"] + [pr["T_out"]]) + "},")
+    lines.append("};")
+    lines.append(f"static __device__ const uint16_t kJac[{nreg}][225] = {{")
+    for _, (kind, pr) in progs:
+        if kind == "jrhs":
+            lines.append("    {" + ", ".join(str(v) for v in pr["jac_out"]) + "},")
+    lines.append("};")
     lines.append(f"}} }}  // namespace wr::coop{G}")
     return "\n".join(lines) + "\n"
 
@@ -1114,15 +1350,27 @@ GEN_DIR = os.path.join(os.path.dirname(HERE), "csrc", "generated")
 LANES_PER_CELL = (8, 16, 32)
 
 
-def emit_all(out_dir: str = GEN_DIR, ir_path: str = ir_io.DEFAULT_PATH) -> list:
+def _emit_one(G: int, out_dir: str, ir_path: str) -> str:
     from .build_network import _write_if_changed
-    dag = ir_io.load(ir_path)
-    digest = ir_io.digest(ir_path)
-    paths = []
-    for G in LANES_PER_CELL:
-        path = os.path.join(out_dir, f"coop_prog_g{G}.h")
-        _write_if_changed(path, emit_header(G, generate(G, dag), digest))
-        paths.append(path)
+    path = os.path.join(out_dir, f"coop_prog_g{G}.h")
+    gen = generate(G, ir_io.load(ir_path), regimes=REGIMES if G in REGIME_LANES else ())
+    _write_if_changed(path, emit_header(G, gen, ir_io.digest(ir_path)))
+    return path
+
+
+def emit_all(out_dir: str = GEN_DIR, ir_path: str = ir_io.DEFAULT_PATH) -> list:
+    """The headers of every lane width, one process each (seconds of scheduling).
+    Nothing is rewritten when they are newer than the generator and network.ir."""
+    paths = [os.path.join(out_dir, f"coop_prog_g{G}.h") for G in LANES_PER_CELL]
+    deps = [os.path.join(HERE, f) for f in ("coop.py", "ir_io.py", "network_dag.py")] + [ir_path]
+    if all(os.path.exists(p) and os.path.getmtime(p) >= max(map(os.path.getmtime, deps)) for p in paths):
+        return paths
+    with concurrent.futures.ThreadPoolExecutor(len(LANES_PER_CELL)) as ex:
+        cmd = "import sys; from warp_reactor_gb300.gen import coop; coop._emit_one(int(sys.argv[1]), *sys.argv[2:])"
+        jobs = [ex.submit(subprocess.run, [sys.executable, "-c", cmd, str(G), out_dir, ir_path], check=True,
+                          cwd=os.path.dirname(os.path.dirname(HERE))) for G in LANES_PER_CELL]
+        for j in jobs:
+            j.result()
     return paths
 
 
