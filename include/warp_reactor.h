@@ -216,7 +216,7 @@ int wr_run_cells(wr_collapse_state* cells, int num_cells, int perturb,
  * or run on a device whose memory is budgeted for them.  This entry point runs
  * one advance step on num_cells <= WR_NOALLOC_MAX_CELLS records in the caller's
  * device memory, updated in place, and allocates nothing: its scratch is one
- * fixed file-scope device array (7.9 MiB, resident on every GPU that loads the
+ * fixed file-scope device array (0.88 MiB, resident on every GPU that loads the
  * library until the process exits).  Its arithmetic is WR_MATH_PORTABLE: the
  * result equals wr_advance of a WR_MATH_PORTABLE context on those cells bit for
  * bit.  Calls share the scratch array, so calls that overlap on the GPU race;
@@ -229,7 +229,7 @@ int wr_run_cells(wr_collapse_state* cells, int num_cells, int perturb,
  * non-blocking streams before the call (cudaStreamSynchronize or an event).
  * No counterpart in the reference. */
 #define WR_NOALLOC_MAX_CELLS 4096
-#define WR_NOALLOC_LANES 4096
+#define WR_NOALLOC_LANES 4096 /* of earlier versions; the scratch no longer depends on it */
 int wr_advance_cells_noalloc(wr_collapse_state* d_cells, int num_cells, int completed_global_steps,
                              double next_grid_time, double dt_grid, int* integrated_out);
 

@@ -35,7 +35,7 @@ NVCC_FLAGS = ARCH + ["-O3", "-std=c++17", "-lineinfo", "--fmad=false", "-Xcompil
                      "-Xcompiler", "-ffp-contract=off", "-I", INCLUDE, "-I", CSRC]
 CXX_FLAGS = ["-O2", "-std=c++17", "-ffp-contract=off", "-fPIC"]
 
-CUDA_UNITS = ["wr_capi.cu", "wr_adv_portable.cu", "wr_adv_cuda.cu", "wr_adv_cta32.cu", "wr_diag.cu", "wr_noalloc.cu",
+CUDA_UNITS = ["wr_capi.cu", "wr_adv_portable.cu", "wr_adv_cuda.cu", "wr_diag.cu", "wr_noalloc.cu",
               "wr_adv_coop8.cu", "wr_adv_coop16.cu", "wr_adv_coop32.cu"]
 # differentiation form: relocatable device code, device-linked into one object
 # (its generated derivative code is split over several units that compile in parallel)

@@ -5,6 +5,7 @@
 // per block: as many as the block's shared memory holds) before this file.
 #include "wr_launch.h"
 #include "wr_coop.cuh"
+#include "wr_coop_cta32.cuh"
 
 #define WR_CAT2(a, b) a##b
 #define WR_CAT(a, b) WR_CAT2(a, b)
@@ -67,6 +68,49 @@ cudaError_t WR_CAT(launch_advance_coop, WR_COOP_G)(int math_cuda, int blocks, cu
     }
     return cudaGetLastError();
 }
+
+// the structured policy's advance at this lane width, a tile on `cluster` SMs
+// (wr_launch.h: cta32_shape picks the pair)
+namespace {
+template <class M, int CL>
+cudaError_t launch_cta32(int tiles, int sms, cudaStream_t stream, DevState s, StepCtl* ctl) {
+    constexpr size_t smem = static_cast<size_t>(kTileCells / CL) * Tab::kNV * 8;
+    static_assert(smem + sizeof(TileCtl<kTileCells / CL>) <= 232448, "a tile's block exceeds 227 KiB of shared memory");
+    auto k = k_advance_cta32<M, kG, CL, Tab>;
+    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(k), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(CL == 1 ? (tiles < sms ? tiles : sms) : tiles * CL));
+    cfg.blockDim = dim3(kTileCells / CL * kG);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = CL;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = CL > 1 ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, k, s, ctl);
+    return e == cudaSuccess ? cudaGetLastError() : e;
+}
+}  // namespace
+#if WR_COOP_G != 8
+cudaError_t WR_CAT(launch_advance_cta32_, WR_COOP_G)(int math_cuda, int cluster, int tiles, int sms,
+                                                     cudaStream_t stream, DevState s, StepCtl* ctl) {
+#if WR_COOP_G == 16
+    (void)cluster;
+    return math_cuda ? launch_cta32<CudaMath, 1>(tiles, sms, stream, s, ctl)
+                     : launch_cta32<PortableMathCall, 1>(tiles, sms, stream, s, ctl);
+#else
+    if (cluster == 4)
+        return math_cuda ? launch_cta32<CudaMath, 4>(tiles, sms, stream, s, ctl)
+                         : launch_cta32<PortableMathCall, 4>(tiles, sms, stream, s, ctl);
+    return math_cuda ? launch_cta32<CudaMath, 2>(tiles, sms, stream, s, ctl)
+                     : launch_cta32<PortableMathCall, 2>(tiles, sms, stream, s, ctl);
+#endif
+}
+#endif
 
 namespace {
 constexpr int kDiagWarps = 4;

@@ -73,8 +73,6 @@ struct wr_ctx {
     unsigned long long* phases = nullptr;  // wr_diag_coop_phases: 16 device counters
     int policy = WR_POLICY_GRIDWIDE_INDEPENDENT;
     double* local_dt = nullptr;  // legacy-local policy: each cell's own dt
-    double* cta_j = nullptr;     // cta32 policy: per-cell Jacobian [225][n]
-    double* cta_e = nullptr;     // cta32 policy: per-cell iteration matrix [225][n]
     cudaEvent_t ev[4 * WR_MAX_COLLAPSE_STEPS + 2] = {};
     int ev_used = 0;
     wr_run_timing timing{};
@@ -218,6 +216,18 @@ __global__ void __launch_bounds__(256) k_commit(DevState s, StepCtl* ctl) {
     }
 }
 
+cudaError_t launch_order_preburn(cudaStream_t stream, DevState s, StepCtl* ctl) {
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    k_order_preburn<<<(s.n + 255) / 256, 256, 0, stream>>>(s, ctl);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_commit(cudaStream_t stream, DevState s, StepCtl* ctl) {
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    k_commit<<<(s.n + 255) / 256, 256, 0, stream>>>(s, ctl);
+    return cudaGetLastError();
+}
+
 // start of an outer step driven by the host (wr_prepare; one grid)
 __global__ void k_begin_step(StepCtl* ctl, int cgs, double grid_time, int step, int perturb) {
     for (int b = 0; b < kBuckets; ++b) ctl->hist[b] = 0;
@@ -348,9 +358,14 @@ bool coop_active(const wr_ctx* ctx) {
 
 cudaError_t launch_advance(wr_ctx* ctx) {
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    if (ctx->policy == WR_POLICY_GRIDWIDE_CTA32)
-        return launch_advance_cta32(ctx->math == WR_MATH_CUDA ? 1 : 0, cta32_blocks(ctx->n), ctx->stream, ctx->s,
-                                    ctx->ctl, ctx->cta_j, ctx->cta_e);
+    if (ctx->policy == WR_POLICY_GRIDWIDE_CTA32) {
+        const int math_cuda = ctx->math == WR_MATH_CUDA ? 1 : 0;
+        const int tiles = (ctx->n + 31) / 32;
+        const Cta32Shape sh = cta32_shape(tiles, ctx->sms);
+        return sh.lanes == 16
+                   ? launch_advance_cta32_16(math_cuda, sh.cluster, tiles, ctx->sms, ctx->stream, ctx->s, ctx->ctl)
+                   : launch_advance_cta32_32(math_cuda, sh.cluster, tiles, ctx->sms, ctx->stream, ctx->s, ctx->ctl);
+    }
     const int blocks = ctx->sms * kAdvanceShapes[ctx->variant].blocks_per_sm;
     if (is_coop(ctx->variant)) {
         const int math_cuda = ctx->math == WR_MATH_CUDA ? 1 : 0;
@@ -367,20 +382,15 @@ cudaError_t launch_advance(wr_ctx* ctx) {
 
 cudaError_t launch_order(wr_ctx* ctx) {
     if (ctx->policy == WR_POLICY_GRIDWIDE_CTA32) return cudaSuccess;  // tiles are fixed: no work queue
+    if (coop_active(ctx)) return launch_order_preburn(ctx->stream, ctx->s, ctx->ctl);
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    if (coop_active(ctx))
-        k_order_preburn<<<(ctx->n + 255) / 256, 256, 0, ctx->stream>>>(ctx->s, ctx->ctl);
-    else
-        k_order<<<(ctx->n + 255) / 256, 256, 0, ctx->stream>>>(ctx->s, ctx->ctl);
+    k_order<<<(ctx->n + 255) / 256, 256, 0, ctx->stream>>>(ctx->s, ctx->ctl);
     return cudaGetLastError();
 }
 
 // after the cooperative advance: commit the cells it burned
 cudaError_t launch_commit(wr_ctx* ctx) {
-    if (!coop_active(ctx)) return cudaSuccess;
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    k_commit<<<(ctx->n + 255) / 256, 256, 0, ctx->stream>>>(ctx->s, ctx->ctl);
-    return cudaGetLastError();
+    return coop_active(ctx) ? launch_commit(ctx->stream, ctx->s, ctx->ctl) : cudaSuccess;
 }
 
 cudaError_t launch_prepare(wr_ctx* ctx) {
@@ -541,8 +551,6 @@ void wr_destroy(wr_ctx* ctx) {
     cudaFree(ctx->jbackup);
     cudaFree(ctx->ebuf);
     cudaFree(ctx->local_dt);
-    cudaFree(ctx->cta_j);
-    cudaFree(ctx->cta_e);
     cudaFree(ctx->dt_hist);
     cudaFree(ctx->staging);
     cudaFree(ctx->phases);
@@ -876,12 +884,6 @@ int wr_set_policy(wr_ctx* ctx, int policy) {
     if (policy == WR_POLICY_LEGACY_LOCAL && !ctx->local_dt) {
         const cudaError_t e = cudaMalloc(&ctx->local_dt, static_cast<size_t>(ctx->n) * sizeof(double));
         if (e != cudaSuccess) return fail("cudaMalloc(local dt)", e);
-    }
-    if (policy == WR_POLICY_GRIDWIDE_CTA32 && !ctx->cta_j) {
-        const size_t bytes = static_cast<size_t>(ctx->n) * NEQ * NEQ * sizeof(double);
-        cudaError_t e = cudaMalloc(&ctx->cta_j, bytes);
-        if (e == cudaSuccess) e = cudaMalloc(&ctx->cta_e, bytes);
-        if (e != cudaSuccess) return fail("wr_set_policy cta32 buffers", e);
     }
     ctx->policy = policy;
     ctx->s.local_dt = policy == WR_POLICY_LEGACY_LOCAL ? ctx->local_dt : nullptr;

@@ -604,6 +604,100 @@ struct PhaseClock<true> {
     }
 };
 
+// One ROS2S attempt (reproducer.cpp:7259-7304) of the warp's cells from y with step h:
+// the candidate state, its error norm, and the factorisation's info (0: regular; the
+// other results then mean nothing).  FMAX: the error scale's maximum by fmax, which
+// drops a NaN (the structured policy), instead of std::max.
+template <class M, int G, class Tab, bool FMAX, int K, class PC>
+__device__ __forceinline__ int ros2s_attempt(uint64_t* V, const double (&y)[K], double h, int& regime, int gl, PC& pc,
+                                             double (&ynew)[K], double& err) {
+    using namespace coop;
+    double* E = reinterpret_cast<double*>(V + kE);
+    double ak1[K], ak2[K], w[K];
+    const int jw = evaluate<M, G, Tab, K>(0, y, regime, gl, V);
+    pc.mark(PH_JPROG);
+    load_outputs<G, K>(V, Tab::out(jw), ak1, gl);
+    gather_matrix<G>(V, Tab::jac(jw / 2), gl);
+    const double fac = ddiv(1.0, h * kGamma);
+#pragma unroll
+    for (int t = 0; t < K; ++t) {
+        const int c = gl + t * G;
+        if (c < NEQ) E[c * NEQ + c] = E[c * NEQ + c] + fac;
+    }
+    __syncwarp();
+    pc.mark(PH_MISC);
+    uint64_t ip = 0;
+    const int info = lu_coop<G>(E, gl, ip);
+    uint64_t rY[K];
+    diag_recips<G, K>(E, rY, gl);
+    pc.mark(PH_LU);
+    solve_coop<G, K>(E, ip, rY, ak1, gl);
+    pc.mark(PH_SOLVE);
+    // stage 2
+    {
+        double yn[K];
+        const double c21h = ddiv(kC21, h);
+#pragma unroll
+        for (int t = 0; t < K; ++t) {
+            yn[t] = y[t] + kA21 * ak1[t];
+            w[t] = c21h * ak1[t];
+        }
+        pc.mark(PH_MISC);
+        const int rw = evaluate<M, G, Tab, K>(1, yn, regime, gl, V);
+        pc.mark(PH_RPROG);
+        double dy[K];
+        load_outputs<G, K>(V, Tab::out(rw), dy, gl);
+#pragma unroll
+        for (int t = 0; t < K; ++t) w[t] += dy[t];
+        pc.mark(PH_MISC);
+        solve_coop<G, K>(E, ip, rY, w, gl);
+        pc.mark(PH_SOLVE);
+#pragma unroll
+        for (int t = 0; t < K; ++t) ak2[t] = w[t];
+    }
+    // stage 3
+    {
+        double yn[K];
+#pragma unroll
+        for (int t = 0; t < K; ++t) {
+            yn[t] = y[t] + kA31 * ak1[t] + kA32 * ak2[t];
+            w[t] = ddiv(kC31 * ak1[t] + kC32 * ak2[t], h);
+        }
+        __syncwarp();  // every lane has read the stage-2 outputs
+        pc.mark(PH_MISC);
+        const int rw = evaluate<M, G, Tab, K>(1, yn, regime, gl, V);
+        pc.mark(PH_RPROG);
+        double dy[K];
+        load_outputs<G, K>(V, Tab::out(rw), dy, gl);
+#pragma unroll
+        for (int t = 0; t < K; ++t) w[t] += dy[t];
+        pc.mark(PH_MISC);
+        solve_coop<G, K>(E, ip, rY, w, gl);
+        pc.mark(PH_SOLVE);
+    }
+    // w = k3: candidate and error estimate, reproducer.cpp:7299-7304
+    double sq[K];
+#pragma unroll
+    for (int t = 0; t < K; ++t) {
+        const int c = gl + t * G;
+        const double ak3 = w[t];
+        ynew[t] = y[t] + kB1 * ak1[t] + kB2 * ak2[t] + ak3;
+        const double wi = kE1 * ak1[t] + kE2 * ak2[t] + kE3 * ak3;
+        const double rtol = c < NS ? kRtolSpec : kRtolEnergy;
+        const double atol = c < NS ? kAtolSpec : kAtolEnergy;
+        const double a = ::fabs(y[t]), b = ::fabs(ynew[t]);
+        const double sk = atol + rtol * (FMAX ? ::fmax(a, b) : smax(a, b));
+        const double term = ddiv(wi, sk);
+        sq[t] = term * term;
+    }
+    // err = sum over components in index order (0.0 + sq[0] == sq[0]: a square)
+    err = get<G, K>(sq, 0);
+#pragma unroll
+    for (int c = 1; c < NEQ; ++c) err = err + get<G, K>(sq, c);
+    err = ::sqrt(ddiv(err, 15.0));
+    return info;
+}
+
 // The cooperative burn: persistent blocks of W warps, G lanes per cell, each group
 // taking cells from the work queue until it is empty.  PH: the phase-counting
 // instantiation (phases: its 16 counters).
@@ -619,7 +713,6 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
     const int gl = lane % G;
     const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (slot * G));
     uint64_t* V = sm + static_cast<size_t>((threadIdx.x >> 5) * SLOTS + slot) * Tab::kNV;
-    double* E = reinterpret_cast<double*>(V + kE);
     init_reserved<M, G, Tab>(V, gl);
     const int n = s.n;
     const unsigned int queued = ctl->queued;
@@ -630,10 +723,9 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
     bool have = false;     // the group holds a cell
     bool drained = false;  // it has seen the queue's end
     int regime = 0;        // the temperature regime of its last evaluation
-    double y[K], f0[K], ak1[K], ak2[K], w[K];
+    double y[K];
 #pragma unroll
-    for (int t = 0; t < K; ++t) y[t] = f0[t] = ak1[t] = ak2[t] = w[t] = 0.0;
-    uint64_t ip = 0;
+    for (int t = 0; t < K; ++t) y[t] = 0.0;
 
 #pragma unroll 1
     while (true) {
@@ -733,91 +825,11 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
         pc.mark(PH_QUEUE);
         pc.attempt();
 
-        // ---- one ROS2S attempt, reproducer.cpp:7259-7345
-        const int jw = evaluate<M, G, Tab, K>(0, y, regime, gl, V);
-        pc.mark(PH_JPROG);
-        load_outputs<G, K>(V, Tab::out(jw), f0, gl);
-        gather_matrix<G>(V, Tab::jac(jw / 2), gl);
         if (L.fresh) L.n_jac += 1;
         L.fresh = false;
         const double h = L.h;
-        const double fac = ddiv(1.0, h * kGamma);
-#pragma unroll
-        for (int t = 0; t < K; ++t) {
-            const int c = gl + t * G;
-            if (c < NEQ) E[c * NEQ + c] = E[c * NEQ + c] + fac;
-        }
-        __syncwarp();
-        pc.mark(PH_MISC);
-        const int info = lu_coop<G>(E, gl, ip);
-        uint64_t rY[K];
-        diag_recips<G, K>(E, rY, gl);
-        pc.mark(PH_LU);
-#pragma unroll
-        for (int t = 0; t < K; ++t) ak1[t] = f0[t];
-        solve_coop<G, K>(E, ip, rY, ak1, gl);
-        pc.mark(PH_SOLVE);
-        // stage 2
-        {
-            double yn[K];
-            const double c21h = ddiv(kC21, h);
-#pragma unroll
-            for (int t = 0; t < K; ++t) {
-                yn[t] = y[t] + kA21 * ak1[t];
-                w[t] = c21h * ak1[t];
-            }
-            pc.mark(PH_MISC);
-            const int rw = evaluate<M, G, Tab, K>(1, yn, regime, gl, V);
-            pc.mark(PH_RPROG);
-            double dy[K];
-            load_outputs<G, K>(V, Tab::out(rw), dy, gl);
-#pragma unroll
-            for (int t = 0; t < K; ++t) w[t] += dy[t];
-            pc.mark(PH_MISC);
-            solve_coop<G, K>(E, ip, rY, w, gl);
-            pc.mark(PH_SOLVE);
-#pragma unroll
-            for (int t = 0; t < K; ++t) ak2[t] = w[t];
-        }
-        // stage 3
-        {
-            double yn[K];
-#pragma unroll
-            for (int t = 0; t < K; ++t) {
-                yn[t] = y[t] + kA31 * ak1[t] + kA32 * ak2[t];
-                w[t] = ddiv(kC31 * ak1[t] + kC32 * ak2[t], h);
-            }
-            __syncwarp();  // every lane has read the stage-2 outputs
-            pc.mark(PH_MISC);
-            const int rw = evaluate<M, G, Tab, K>(1, yn, regime, gl, V);
-            pc.mark(PH_RPROG);
-            double dy[K];
-            load_outputs<G, K>(V, Tab::out(rw), dy, gl);
-#pragma unroll
-            for (int t = 0; t < K; ++t) w[t] += dy[t];
-            pc.mark(PH_MISC);
-            solve_coop<G, K>(E, ip, rY, w, gl);
-            pc.mark(PH_SOLVE);
-        }
-        // w = k3: candidate and error estimate, reproducer.cpp:7299-7304
-        double ynew[K], sq[K];
-#pragma unroll
-        for (int t = 0; t < K; ++t) {
-            const int c = gl + t * G;
-            const double ak3 = w[t];
-            ynew[t] = y[t] + kB1 * ak1[t] + kB2 * ak2[t] + ak3;
-            const double wi = kE1 * ak1[t] + kE2 * ak2[t] + kE3 * ak3;
-            const double rtol = c < NS ? kRtolSpec : kRtolEnergy;
-            const double atol = c < NS ? kAtolSpec : kAtolEnergy;
-            const double sk = atol + rtol * smax(::fabs(y[t]), ::fabs(ynew[t]));
-            const double term = ddiv(wi, sk);
-            sq[t] = term * term;
-        }
-        // err = sum over components in index order (0.0 + sq[0] == sq[0]: a square)
-        double err = get<G, K>(sq, 0);
-#pragma unroll
-        for (int c = 1; c < NEQ; ++c) err = err + get<G, K>(sq, c);
-        err = ::sqrt(ddiv(err, 15.0));
+        double ynew[K], err;
+        const int info = ros2s_attempt<M, G, Tab, false, K>(V, y, h, regime, gl, pc, ynew, err);
         // step-size controller, reproducer.cpp:7308-7344
         const double raw_fac = ddiv(StepMath<M>::cbrt(err), kSafe);
         const double fac_step = smax(1.0 / kFacMax, smin(1.0 / kFacMin, raw_fac));

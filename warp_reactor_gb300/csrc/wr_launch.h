@@ -61,11 +61,20 @@ cudaError_t launch_advance_portable(int variant, int blocks, cudaStream_t stream
 cudaError_t launch_advance_cuda(int variant, int blocks, cudaStream_t stream, DevState s, StepCtl* ctl,
                                 double* jbackup, double* ebuf);
 cudaError_t configure_advance_portable();
-// gridwide-structured-cta32 policy (wr_adv_cta32.cu): one warp per 32-cell tile;
-// jall / eall are per-cell [225][n] Jacobian and iteration-matrix arrays
-cudaError_t launch_advance_cta32(int math_cuda, int blocks, cudaStream_t stream, DevState s, StepCtl* ctl,
-                                 double* jall, double* eall);
-int cta32_blocks(int n);
+// gridwide-structured-cta32 policy (wr_coop_cta32.cuh): a tile of 32 cells on a cluster
+// of `cluster` SMs at `lanes` lanes per cell.  A trial's latency sets the time while
+// there are SMs to spare, so a tile spreads over four SMs (8 cells each) or two as long
+// as that takes no second wave; beyond that one SM per tile at 16 lanes per cell.
+struct Cta32Shape {
+    int lanes, cluster;
+};
+constexpr Cta32Shape cta32_shape(int tiles, int sms) {
+    return tiles * 4 <= sms ? Cta32Shape{32, 4} : tiles * 2 <= sms ? Cta32Shape{32, 2} : Cta32Shape{16, 1};
+}
+cudaError_t launch_advance_cta32_16(int math_cuda, int cluster, int tiles, int sms, cudaStream_t stream, DevState s,
+                                    StepCtl* ctl);
+cudaError_t launch_advance_cta32_32(int math_cuda, int cluster, int tiles, int sms, cudaStream_t stream, DevState s,
+                                    StepCtl* ctl);
 cudaError_t configure_advance_cuda();
 // cooperative advance (wr_adv_coop<G>.cu): G lanes per cell, one block per SM
 cudaError_t configure_advance_coop8();
@@ -77,6 +86,10 @@ cudaError_t launch_advance_coop16(int math_cuda, int blocks, cudaStream_t stream
                                   unsigned long long* phases);
 cudaError_t launch_advance_coop32(int math_cuda, int blocks, cudaStream_t stream, DevState s, StepCtl* ctl,
                                   unsigned long long* phases);
+// around the cooperative advance (wr_capi.cu): the queue with the advance's prologue,
+// and the commit of the cells it burned
+cudaError_t launch_order_preburn(cudaStream_t stream, DevState s, StepCtl* ctl);
+cudaError_t launch_commit(cudaStream_t stream, DevState s, StepCtl* ctl);
 // diagnostics of the cooperative programs and LU on device buffers (wr_diag.cu)
 cudaError_t diag_coop_network8(int math_cuda, int n, const double* y, double* J, double* f, double* f2);
 cudaError_t diag_coop_network16(int math_cuda, int n, const double* y, double* J, double* f, double* f2);

@@ -1191,9 +1191,9 @@ def generate(G: int, dag=None, limit="default", tune="default", banked="default"
     first = RES_BASE + len(rconst) + len(rfun)
     if banked == "default":
         banked = G in BANKED
-    # slot count (write sink included) that keeps the block's warps, one below the
-    # block's whole shared memory
-    cap = max(nv for nv in range(first, MAX_SLOTS) if warps_per_block(G, nv) == MAX_WARPS) - 1
+    # slot count (write sink included) that keeps the block's warps and leaves room
+    # for the tile controller's shared words (wr_coop_cta32.cuh)
+    cap = max(nv for nv in range(first, MAX_SLOTS) if warps_per_block(G, nv) == MAX_WARPS) - 5
     scheds = {}
     for (reg, kind), (P, out) in built.items():
         key = kind if reg is None else (REGIMES.index(reg) + 1, kind)
