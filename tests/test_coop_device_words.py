@@ -14,7 +14,7 @@ from warp_reactor_gb300.gen import coop, ir_io
 
 
 def slow(cls, x, y, fl, oracle):
-    if cls == C_DIV:
+    if cls in (C_DIV, coop.C_GDIV):
         x = (x & ABS) if fl & coop.DV_ABS else x
         x = (x ^ SIGN) if fl & coop.DV_NEG else x
         num, den = (d(y), d(x)) if fl & coop.DV_SWAP else (d(x), d(y))
@@ -61,6 +61,10 @@ def overlapped(words, ctl, V, oracle):
             dst = (m >> 48) & 0xffff
             if cls == C_FMA:
                 results.append((dst >> 3, u(fma(d(x), d(y), d(z)))))
+            elif cls == coop.C_GMUL:
+                results.append((dst >> 3, 0 if x & ABS == 0 else u(d(x) * d(y))))
+            elif cls == coop.C_GDIV and x & ABS == 0:
+                results.append((dst >> 3, 0))
             elif cls != C_NONE:
                 results.append((dst >> 3, u(slow(cls, x, y, dst & 7, oracle))))
             else:

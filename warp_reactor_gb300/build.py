@@ -36,10 +36,7 @@ NVCC_FLAGS = ARCH + ["-O3", "-std=c++17", "-lineinfo", "--fmad=false", "-Xcompil
 CXX_FLAGS = ["-O2", "-std=c++17", "-ffp-contract=off", "-fPIC"]
 
 CUDA_UNITS = ["wr_capi.cu", "wr_adv_portable.cu", "wr_adv_cuda.cu", "wr_diag.cu", "wr_noalloc.cu",
-              "wr_adv_coop8.cu", "wr_adv_coop16.cu", "wr_adv_coop32.cu"]
-# differentiation form: relocatable device code, device-linked into one object
-# (its generated derivative code is split over several units that compile in parallel)
-RDC_UNITS = ["wr_diff.cu", "wr_diff_bwd.cu", "wr_diff_net.cu", "wr_diff_jvjp0.cu", "wr_diff_jvjp1.cu"]
+              "wr_adv_coop8.cu", "wr_adv_coop16.cu", "wr_adv_coop32.cu", "wr_diff.cu", "wr_diff_coop.cu"]
 
 
 def _nvcc() -> str:
@@ -85,25 +82,17 @@ def build_library(verbose=False, jobs=None) -> str:
     headers = _headers()
     objs = []
     tasks = []
-    rdc_objs = []
-    for unit in CUDA_UNITS + RDC_UNITS:
+    for unit in CUDA_UNITS:
         src = os.path.join(CSRC, unit)
         obj = os.path.join(OUT, unit.replace(".cu", ".o"))
-        rdc = unit in RDC_UNITS
-        (rdc_objs if rdc else objs).append(obj)
+        objs.append(obj)
         if _stale(obj, [src] + headers):
-            tasks.append([nvcc] + NVCC_FLAGS + (["-rdc=true"] if rdc else []) + ["-c", src, "-o", obj])
-    # longest units first
-    tasks.sort(key=lambda c: 0 if any(u in c[-3] for u in ("jvjp", "bwd", "net")) else 1)
-    with cf.ThreadPoolExecutor(max_workers=jobs or len(CUDA_UNITS) + len(RDC_UNITS)) as ex:
+            tasks.append([nvcc] + NVCC_FLAGS + ["-c", src, "-o", obj])
+    with cf.ThreadPoolExecutor(max_workers=jobs or len(CUDA_UNITS)) as ex:
         list(ex.map(lambda c: _run(c, verbose), tasks))
-    dlink = os.path.join(OUT, "wr_diff_dlink.o")
-    if _stale(dlink, rdc_objs):
-        _run([nvcc] + ARCH + ["-dlink", "-Xcompiler", "-fPIC", "-o", dlink] + rdc_objs, verbose)
     lib = os.path.join(OUT, "libwarp_reactor.so")
-    all_objs = objs + rdc_objs + [dlink]
-    if _stale(lib, all_objs):
-        _run([nvcc] + ARCH + ["-shared", "-o", lib] + all_objs + ["-lcudart"], verbose)
+    if _stale(lib, objs):
+        _run([nvcc] + ARCH + ["-shared", "-o", lib] + objs + ["-lcudart"], verbose)
     return lib
 
 

@@ -20,6 +20,7 @@ struct Tab {
     static constexpr int kNR = cp::kNR;
     static constexpr int kNF = cp::kNF;
     static constexpr int kRegimes = cp::kRegimes;
+    static constexpr bool kAdjoint = false;
     static __device__ __forceinline__ const uint64_t* vconst() { return cp::kVConst; }
     static __device__ __forceinline__ const ulonglong2* vfun() { return cp::kVFun; }
     static __device__ __forceinline__ const ulonglong2* prog() { return cp::kProg; }

@@ -490,15 +490,8 @@ int wr_create_batch(int num_grids, const int* cells_per_grid, int device, int ma
     ctx->sms = sms > 0 ? sms : 1;
     ctx->advance_blocks = ctx->sms;
     ctx->variant = default_variant(num_cells, ctx->sms);
-    size_t nslots = 0;  // lane slots of the largest configuration
-    for (const AdvanceShape& sh : kAdvanceShapes) {
-        const size_t slots = static_cast<size_t>(ctx->sms) * sh.blocks_per_sm * sh.threads;
-        nslots = slots > nslots ? slots : nslots;
-    }
     e = cudaMalloc(&ctx->state_buf, bytes);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->ctl, sizeof(StepCtl) * ctx->G);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->jbackup, nslots * NEQ * NEQ * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->ebuf, nslots * NEQ * NEQ * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->dt_hist, static_cast<size_t>(ctx->G) * WR_MAX_COLLAPSE_STEPS * sizeof(double));
     if (e == cudaSuccess) e = cudaMallocHost(&ctx->host_ctl, sizeof(StepCtl) * ctx->G);
     if (e == cudaSuccess) e = ctx->math == WR_MATH_CUDA ? configure_advance_cuda() : configure_advance_portable();
@@ -563,6 +556,22 @@ static int ensure_staging(wr_ctx* ctx) {
     if (ctx->staging) return WR_SUCCESS;
     const cudaError_t e = cudaMalloc(&ctx->staging, static_cast<size_t>(ctx->n) * sizeof(wr_collapse_state));
     return e == cudaSuccess ? WR_SUCCESS : fail("cudaMalloc(staging)", e);
+}
+
+// the lane-per-cell shapes' Jacobian backup and iteration matrices, allocated when one
+// of these shapes is first chosen (two times 105 MB that the cooperative advance never
+// touches: half the time of a context's creation)
+static int ensure_lane_scratch(wr_ctx* ctx) {
+    if (ctx->ebuf) return WR_SUCCESS;
+    size_t nslots = 0;  // lane slots of the largest configuration
+    for (const AdvanceShape& sh : kAdvanceShapes) {
+        const size_t slots = static_cast<size_t>(ctx->sms) * sh.blocks_per_sm * sh.threads;
+        nslots = slots > nslots ? slots : nslots;
+    }
+    const size_t bytes = nslots * NEQ * NEQ * sizeof(double);
+    cudaError_t e = ctx->jbackup ? cudaSuccess : cudaMalloc(&ctx->jbackup, bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->ebuf, bytes);
+    return e == cudaSuccess ? WR_SUCCESS : fail("cudaMalloc(lane scratch)", e);
 }
 
 int wr_upload(wr_ctx* ctx, const wr_collapse_state* cells) {
@@ -829,6 +838,7 @@ int wr_grid_dt_history(wr_ctx* ctx, int grid, double* out, int max_steps) {
 int wr_autotune(wr_ctx* ctx, int perturb, int steps, int* best_variant) {
     if (!ctx || !best_variant || steps < 1) return fail_msg("wr_autotune: bad argument");
     int rc = set_device(ctx);
+    if (rc == WR_SUCCESS) rc = ensure_lane_scratch(ctx);  // it times the lane-per-cell shapes too
     if (rc != WR_SUCCESS) return rc;
     const size_t bytes = static_cast<size_t>(ctx->n) * ((3 + NS + 2) * sizeof(double) + 7 * sizeof(uint64_t) + 4 * sizeof(int));
     void* snap = nullptr;
@@ -893,6 +903,11 @@ int wr_set_policy(wr_ctx* ctx, int policy) {
 int wr_set_advance_variant(wr_ctx* ctx, int variant) {
     if (!ctx) return fail_msg("wr_set_advance_variant: null context");
     if (variant < 0 || variant >= kAdvanceVariants) return fail_msg("wr_set_advance_variant: unknown variant");
+    if (!is_coop(variant)) {
+        int rc = set_device(ctx);
+        if (rc == WR_SUCCESS) rc = ensure_lane_scratch(ctx);
+        if (rc != WR_SUCCESS) return rc;
+    }
     ctx->variant = variant;
     return WR_SUCCESS;
 }

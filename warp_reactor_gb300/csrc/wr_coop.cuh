@@ -50,6 +50,9 @@ constexpr int kQBurnOK = -4;   // burned successfully: k_commit commits it
 namespace coop {
 
 enum { C_NONE = 0, C_FMA = 1, C_EXP = 2, C_LOG = 3, C_SQRT = 4, C_DIV = 5 };
+// classes of derivative programs only (tables with Tab::kAdjoint): V[X] V[Y] and
+// V[X] / V[Y], which are 0 where V[X] is zero, whatever V[Y] holds
+enum { C_GMUL = 6, C_GDIV = 7 };
 enum { I_SEL = 0, I_LE = 1, I_LT = 2, I_SGN = 3 };
 // control byte of a step: class | CTL_INT (it has integer nodes) | CTL_SPECIAL (they
 // include comparisons or sign operations) | CTL_FLUSH (its main results are stored in
@@ -129,7 +132,8 @@ struct StepMath {
 // modifier flags of D
 template <class M>
 __device__ __noinline__ uint64_t slow_step(uint32_t cls, uint64_t x, uint64_t y, uint32_t fl) {
-    if (cls == C_DIV) {
+    if (cls == C_DIV || cls == C_GDIV) {
+        if (cls == C_GDIV && (x & kAbs) == 0) return 0;
         x = (fl & DV_ABS) ? (x & kAbs) : x;
         x = (fl & DV_NEG) ? (x ^ kSign) : x;
         const bool sw = (fl & DV_SWAP) != 0;
@@ -227,6 +231,8 @@ __device__ __noinline__ void run_prog(int which, int gl, uint64_t* V) {
         uint64_t r = 0;
         if (cls == C_FMA)
             r = bits(__fma_rn(dbl(x), dbl(y), dbl(z)));
+        else if (Tab::kAdjoint && cls == C_GMUL)
+            r = (x & kAbs) == 0 ? 0 : bits(__fma_rn(dbl(x), dbl(y), dbl(z)));
         else if (cls != C_NONE)
             r = slow_step<M>(cls, x, y, w1 >> 16);
         if (c & CTL_INT) int_step(c, e.y, vb);
@@ -554,7 +560,7 @@ __device__ __forceinline__ void gather_matrix(uint64_t* V, const uint16_t* jac, 
 
 // Generated tables of one G, supplied by the translation unit that includes the
 // generated header (one unit per G keeps the large initialisers apart).
-//   Tab::kNV, Tab::kNR, Tab::kNF, Tab::kRegimes and device accessors vconst(),
+//   Tab::kNV, Tab::kNR, Tab::kNF, Tab::kRegimes, Tab::kAdjoint and device accessors vconst(),
 //   vfun(), prog(), lit(), ctl(i) (control bytes of four steps), first(w) and steps(w)
 //   of program w = 2 * regime + kind, out(w) (RHS operands, then T), jac(regime) and
 //   regime(k, 0 or 1) (the temperatures between which regime k holds).
@@ -604,16 +610,15 @@ struct PhaseClock<true> {
     }
 };
 
-// One ROS2S attempt (reproducer.cpp:7259-7304) of the warp's cells from y with step h:
-// the candidate state, its error norm, and the factorisation's info (0: regular; the
-// other results then mean nothing).  FMAX: the error scale's maximum by fmax, which
-// drops a NaN (the structured policy), instead of std::max.
-template <class M, int G, class Tab, bool FMAX, int K, class PC>
-__device__ __forceinline__ int ros2s_attempt(uint64_t* V, const double (&y)[K], double h, int& regime, int gl, PC& pc,
-                                             double (&ynew)[K], double& err) {
+// The stages of one ROS2S attempt (reproducer.cpp:7259-7304) of the warp's cells from y
+// with step h: the factorised iteration matrix in the matrix slots, its pivots, k1, k2
+// and k3.  Returns the factorisation's info (0: regular; the rest means nothing
+// otherwise).
+template <class M, int G, class Tab, int K, class PC>
+__device__ __forceinline__ int ros2s_stages(uint64_t* V, const double (&y)[K], double h, int& regime, int gl, PC& pc,
+                                            uint64_t& ip, double (&ak1)[K], double (&ak2)[K], double (&w)[K]) {
     using namespace coop;
     double* E = reinterpret_cast<double*>(V + kE);
-    double ak1[K], ak2[K], w[K];
     const int jw = evaluate<M, G, Tab, K>(0, y, regime, gl, V);
     pc.mark(PH_JPROG);
     load_outputs<G, K>(V, Tab::out(jw), ak1, gl);
@@ -626,7 +631,7 @@ __device__ __forceinline__ int ros2s_attempt(uint64_t* V, const double (&y)[K], 
     }
     __syncwarp();
     pc.mark(PH_MISC);
-    uint64_t ip = 0;
+    ip = 0;
     const int info = lu_coop<G>(E, gl, ip);
     uint64_t rY[K];
     diag_recips<G, K>(E, rY, gl);
@@ -675,14 +680,22 @@ __device__ __forceinline__ int ros2s_attempt(uint64_t* V, const double (&y)[K], 
         solve_coop<G, K>(E, ip, rY, w, gl);
         pc.mark(PH_SOLVE);
     }
-    // w = k3: candidate and error estimate, reproducer.cpp:7299-7304
+    return info;
+}
+
+// The candidate state from the stages and its error norm (reproducer.cpp:7299-7304).
+// FMAX: the error scale's maximum by fmax, which drops a NaN (the structured policy),
+// instead of std::max.
+template <int G, bool FMAX, int K>
+__device__ __forceinline__ void ros2s_candidate(const double (&y)[K], const double (&ak1)[K], const double (&ak2)[K],
+                                                const double (&ak3)[K], int gl, double (&ynew)[K], double& err) {
+    using namespace coop;
     double sq[K];
 #pragma unroll
     for (int t = 0; t < K; ++t) {
         const int c = gl + t * G;
-        const double ak3 = w[t];
-        ynew[t] = y[t] + kB1 * ak1[t] + kB2 * ak2[t] + ak3;
-        const double wi = kE1 * ak1[t] + kE2 * ak2[t] + kE3 * ak3;
+        ynew[t] = y[t] + kB1 * ak1[t] + kB2 * ak2[t] + ak3[t];
+        const double wi = kE1 * ak1[t] + kE2 * ak2[t] + kE3 * ak3[t];
         const double rtol = c < NS ? kRtolSpec : kRtolEnergy;
         const double atol = c < NS ? kAtolSpec : kAtolEnergy;
         const double a = ::fabs(y[t]), b = ::fabs(ynew[t]);
@@ -695,6 +708,16 @@ __device__ __forceinline__ int ros2s_attempt(uint64_t* V, const double (&y)[K], 
 #pragma unroll
     for (int c = 1; c < NEQ; ++c) err = err + get<G, K>(sq, c);
     err = ::sqrt(ddiv(err, 15.0));
+}
+
+// One attempt: candidate state, error norm, and the factorisation's info
+template <class M, int G, class Tab, bool FMAX, int K, class PC>
+__device__ __forceinline__ int ros2s_attempt(uint64_t* V, const double (&y)[K], double h, int& regime, int gl, PC& pc,
+                                             double (&ynew)[K], double& err) {
+    uint64_t ip;
+    double ak1[K], ak2[K], ak3[K];
+    const int info = ros2s_stages<M, G, Tab, K>(V, y, h, regime, gl, pc, ip, ak1, ak2, ak3);
+    ros2s_candidate<G, FMAX, K>(y, ak1, ak2, ak3, gl, ynew, err);
     return info;
 }
 

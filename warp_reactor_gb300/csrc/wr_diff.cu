@@ -1,5 +1,5 @@
-// wr_diff.cu -- differentiation form: forward kernel and C ABI (the map and its
-// storage are described in wr_diff.cuh).
+// wr_diff.cu -- differentiation form: C ABI (the map and its storage are described in
+// wr_diff.cuh, the kernels are in wr_diff_coop.cu).
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -9,218 +9,6 @@
 
 namespace wr {
 namespace diff {
-
-// ---------------------------------------------------------------- forward pieces
-// ---------------------------------------------------------------- forward pieces
-// One ROS2S attempt (reproducer.cpp:7259-7304) from y with step h and iteration
-// matrix already factorised in E/ip; writes ynew and the error vector.
-__device__ void ros2s_stages(const double* y, double h, MatL E, uint64_t ip, const double* mult,
-                                             double* ak1, double* ak2, double* ak3, double* ynew, double* work) {
-    double X[NS], T, dy[NEQ];
-    state_from_y(y, X, T);
-    net_rhs(X, T, mult, ak1);
-    lu_solve(E, ip, ak1);
-#pragma unroll
-    for (int i = 0; i < NEQ; ++i) {
-        ynew[i] = y[i] + kA21 * ak1[i];
-        ak2[i] = ddiv(kC21, h) * ak1[i];
-    }
-    state_from_y(ynew, X, T);
-    net_rhs(X, T, mult, dy);
-#pragma unroll
-    for (int i = 0; i < NEQ; ++i) ak2[i] += dy[i];
-    lu_solve(E, ip, ak2);
-#pragma unroll
-    for (int i = 0; i < NEQ; ++i) {
-        ynew[i] = y[i] + kA31 * ak1[i] + kA32 * ak2[i];
-        ak3[i] = ddiv(kC31 * ak1[i] + kC32 * ak2[i], h);
-    }
-    state_from_y(ynew, X, T);
-    net_rhs(X, T, mult, dy);
-#pragma unroll
-    for (int i = 0; i < NEQ; ++i) ak3[i] += dy[i];
-    lu_solve(E, ip, ak3);
-#pragma unroll
-    for (int i = 0; i < NEQ; ++i) {
-        ynew[i] = y[i] + kB1 * ak1[i] + kB2 * ak2[i] + ak3[i];
-        work[i] = kE1 * ak1[i] + kE2 * ak2[i] + kE3 * ak3[i];
-    }
-}
-
-__device__ int factor(const double* J, double h, MatL E, uint64_t& ip) {
-    const double fac = ddiv(1.0, h * kGamma);
-#pragma unroll 1
-    for (int r = 0; r < NEQ; ++r)
-#pragma unroll 1
-        for (int c = 0; c < NEQ; ++c) E(r, c) = -J[r * NEQ + c];
-#pragma unroll 1
-    for (int i = 0; i < NEQ; ++i) E(i, i) = E(i, i) + fac;
-    return lu_decompose(E, ip);
-}
-
-// RODAS::integrate with the configure_ros2s settings (:7205-7347, :7582-7590),
-// appending accepted step sizes to h_out (at most cap_left).  Returns the
-// IntegratorResult; *count = accepted steps.
-static __device__ __noinline__ int burn_record(double* y, double tout, const double* mult, double* h_out, int cap_left, int* count) {
-    double Jm[NEQ * NEQ], Em[NEQ * NEQ];
-    MatL E{Em};
-    uint64_t ip = 0;
-    double ak1[NEQ], ak2[NEQ], ak3[NEQ], ynew[NEQ], work[NEQ];
-    const double hmaxn = tout;
-    double h = tout;
-    if (::fabs(h) <= 10.0 * kUround) h = 1.e-6;
-    h = smin(::fabs(h), hmaxn);
-    bool reject = false, last = false;
-    int nsing = 0, n_step = 0, n_accept = 0;
-    double hacc = 0.0, erracc = 1.0, x = 0.0;
-    *count = 0;
-    for (;;) {
-        if (n_step > kMaxSteps) return WR_TOO_MANY_STEPS;
-        if (0.1 * ::fabs(h) <= ::fabs(x) * kUround) return WR_DT_UNDERFLOW;
-        if (last) return WR_SUCCESS;
-        if (x + h * 1.0001 >= tout) {
-            h = tout - x;
-            last = true;
-        }
-        {
-            double X[NS], T;
-            state_from_y(y, X, T);
-            net_jac(X, T, Jm);
-        }
-        for (;;) {
-            if (factor(Jm, h, E, ip) != 0) {
-                nsing += 1;
-                if (nsing >= 5) return WR_LU_DECOMPOSITION_ERROR;
-                h = h * 0.5;
-                reject = true;
-                last = false;
-                continue;
-            }
-            ros2s_stages(y, h, E, ip, mult, ak1, ak2, ak3, ynew, work);
-            n_step += 1;
-            double err = 0.0;
-#pragma unroll
-            for (int i = 0; i < NEQ; ++i) {
-                const double rtol = i < NS ? kRtolSpec : kRtolEnergy;
-                const double atol = i < NS ? kAtolSpec : kAtolEnergy;
-                const double sk = atol + rtol * smax(::fabs(y[i]), ::fabs(ynew[i]));
-                const double term = ddiv(work[i], sk);
-                err += term * term;
-            }
-            err = ::sqrt(ddiv(err, 15.0));
-            const double raw_fac = ddiv(M::cbrt(err), kSafe);
-            const double fac_step = smax(1.0 / kFacMax, smin(1.0 / kFacMin, raw_fac));
-            double hnew = ddiv(h, fac_step);
-            if (err <= 1.0) {
-                n_accept += 1;
-                if (n_accept > 1) {
-                    const double facgus = smax(1.0 / kFacMax,
-                        smin(1.0 / kFacMin, ddiv(ddiv(hacc, h) * M::cbrt(ddiv(err * err, erracc)), kSafe)));
-                    hnew = ddiv(h, smax(fac_step, facgus));
-                }
-                hacc = h;
-                erracc = smax(1.e-2, err);
-                if (*count >= cap_left) return WR_TOO_MANY_STEPS;
-                h_out[*count] = h;
-                *count += 1;
-#pragma unroll
-                for (int i = 0; i < NEQ; ++i) y[i] = ynew[i];
-                x += h;
-                if (::fabs(hnew) > hmaxn) hnew = hmaxn;
-                if (reject) hnew = smin(::fabs(hnew), ::fabs(h));
-                reject = false;
-                h = hnew;
-                break;
-            }
-            reject = true;
-            last = false;
-            h = hnew;
-            if (hnew == 0.0) return WR_DT_UNDERFLOW;  // the reject loop's only other exit
-        }
-    }
-}
-
-// one accepted step of the frozen controller
-__device__ void step_replay(double* y, double h, const double* mult, double* st) {
-    double Jm[NEQ * NEQ], Em[NEQ * NEQ];
-    MatL E{Em};
-    uint64_t ip = 0;
-    double ak1[NEQ], ak2[NEQ], ak3[NEQ], ynew[NEQ], work[NEQ];
-    double X[NS], T;
-    state_from_y(y, X, T);
-    net_jac(X, T, Jm);
-    factor(Jm, h, E, ip);
-    ros2s_stages(y, h, E, ip, mult, ak1, ak2, ak3, ynew, work);
-    if (st != nullptr) {
-        // what the step's adjoint needs: the factorised matrix, pivots, stage vectors
-#pragma unroll 1
-        for (int k = 0; k < NEQ * NEQ; ++k) st[k] = Em[k];
-        st[kStageIp] = __longlong_as_double(static_cast<long long>(ip));
-#pragma unroll
-        for (int i = 0; i < NEQ; ++i) {
-            st[kStageK1 + i] = ak1[i];
-            st[kStageK2 + i] = ak2[i];
-            st[kStageK3 + i] = ak3[i];
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < NEQ; ++i) y[i] = ynew[i];
-}
-
-__global__ void __launch_bounds__(kThreads) k_diff_forward(Args a) {
-    const int i = blockIdx.x * kThreads + threadIdx.x;
-    if (i >= a.n) return;
-    CellS c;
-    {
-        const wr_collapse_state& st = a.cells[i];
-#pragma unroll
-        for (int k = 0; k < NS; ++k) c.xn[k] = a.u ? a.u[15 * i + k] : st.xn[k];
-        c.T = a.u ? a.u[15 * i + NS] : st.T;
-        c.e = st.e;
-        c.rho = st.rho;
-        c.driver = st.density_driver;
-    }
-    double* hrow = a.hbuf + static_cast<size_t>(i) * a.cap;
-    int used = 0;
-    int status = WR_SUCCESS;
-    bool live = true;
-    for (int s = 0; s < a.nsteps; ++s) {
-        unsigned char kind = 0;
-        int cnt = 0;
-        if (live) {
-            save_ckpt(a, s, i, c);
-            double dt;
-            int k = prepare_part(a, s, i, c, dt);
-            if (k == 3) {
-                double y[NEQ];
-                k = advance_part(a.dt_hist[s], dt, c, y);
-                if (k == 3) {
-                    const int r = burn_record(y, a.dt_hist[s], a.mult, hrow + used, a.cap - used, &cnt);
-                    if (r != WR_SUCCESS) {
-                        status = r;
-                        live = false;
-                    } else {
-                        commit_part(c, y);
-                        used += cnt;
-                    }
-                }
-            }
-            if (k < 0) {
-                status = WR_BAD_INPUTS;
-                live = false;
-            } else {
-                kind = static_cast<unsigned char>(k);
-                if (k != 3) live = false;
-            }
-        }
-        a.kind[static_cast<size_t>(s) * a.n + i] = kind;
-        a.counts[static_cast<size_t>(s) * a.n + i] = cnt;
-    }
-#pragma unroll
-    for (int k = 0; k < NS; ++k) a.q[15 * i + k] = c.xn[k];
-    a.q[15 * i + NS] = c.T;
-    a.status[i] = status;
-}
 
 __global__ void k_diff_mult(const double* logm, double* mult) {
     const int r = threadIdx.x;
@@ -232,6 +20,7 @@ __global__ void k_diff_reduce(const double* mbar, const double* mult, int n, dou
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= NP) return;
     double acc = 0.0;
+#pragma unroll 16  // the sums are serial, their loads need not be
     for (int i = 0; i < n; ++i) acc += mbar[static_cast<size_t>(i) * NP + r];
     pbar[r] = acc * mult[r];
 }
@@ -242,7 +31,7 @@ __global__ void k_diff_reduce(const double* mbar, const double* mult, int n, dou
 // ------------------------------------------------------------------ C-ABI
 struct wr_diff {
     int n = 0, max_steps = 0, cap = 0, nseg = 0, device = 0;
-    int nsteps = 0, perturb = 0;
+    int nsteps = 0, perturb = 0, sms = 1;
     bool have_forward = false;
     cudaStream_t stream = nullptr;
     double* ckpt = nullptr;
@@ -256,6 +45,7 @@ struct wr_diff {
     double* mult = nullptr;
     double* dt_hist = nullptr;
     int* status = nullptr;
+    int* queue = nullptr;
     const wr_collapse_state* cells = nullptr;  // the caller's records of the last forward
     const double* u = nullptr;
     std::string error;
@@ -294,6 +84,7 @@ wr::diff::Args make_args(wr_diff* d) {
     a.stage = d->stage;
     a.mbar = d->mbar;
     a.status = d->status;
+    a.queue = d->queue;
     return a;
 }
 
@@ -325,7 +116,9 @@ wr_diff* wr_diff_create(int num_cells, int max_outer_steps, int max_accepted_per
               cuda_ok(d, cudaMalloc(&d->mbar, n * wr::diff::NP * sizeof(double)), "cudaMalloc") &&
               cuda_ok(d, cudaMalloc(&d->mult, wr::diff::NP * sizeof(double)), "cudaMalloc") &&
               cuda_ok(d, cudaMalloc(&d->dt_hist, S * sizeof(double)), "cudaMalloc") &&
-              cuda_ok(d, cudaMalloc(&d->status, n * sizeof(int)), "cudaMalloc");
+              cuda_ok(d, cudaMalloc(&d->status, n * sizeof(int)), "cudaMalloc") &&
+              cuda_ok(d, cudaMalloc(&d->queue, sizeof(int)), "cudaMalloc") &&
+              cuda_ok(d, cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, device), "device query");
     if (!ok) {
         fprintf(stderr, "wr_diff_create: %s\n", d->error.c_str());
         wr_diff_destroy(d);
@@ -347,6 +140,7 @@ void wr_diff_destroy(wr_diff* d) {
     cudaFree(d->mult);
     cudaFree(d->dt_hist);
     cudaFree(d->status);
+    cudaFree(d->queue);
     if (d->stream) cudaStreamDestroy(d->stream);
     delete d;
 }
@@ -372,9 +166,7 @@ int wr_diff_forward(wr_diff* d, const wr_collapse_state* d_cells, const double* 
     wr::diff::k_diff_mult<<<1, 64, 0, d->stream>>>(d_log_mult, d->mult);
     wr::diff::Args a = make_args(d);
     a.q = d_q;
-    const int blocks = (d->n + wr::diff::kThreads - 1) / wr::diff::kThreads;
-    wr::diff::k_diff_forward<<<blocks, wr::diff::kThreads, 0, d->stream>>>(a);
-    if (!cuda_ok(d, cudaGetLastError(), "k_diff_forward launch")) return WR_BAD_INPUTS;
+    if (!cuda_ok(d, wr::diff::launch_diff_forward(a, d->sms, d->stream), "k_diff_forward launch")) return WR_BAD_INPUTS;
     if (!cuda_ok(d, cudaStreamSynchronize(d->stream), "k_diff_forward")) return WR_BAD_INPUTS;
     // first failing cell in index order decides the result
     int* st = new int[d->n];
@@ -399,9 +191,8 @@ int wr_diff_backward(wr_diff* d, const double* d_qbar, double* d_ubar, double* d
     wr::diff::Args a = make_args(d);
     a.qbar = d_qbar;
     a.ubar = d_ubar;
-    const int blocks = (d->n + wr::diff::kThreads - 1) / wr::diff::kThreads;
-    wr::diff::k_diff_backward<<<blocks, wr::diff::kThreads, 0, d->stream>>>(a);
-    if (!cuda_ok(d, cudaGetLastError(), "k_diff_backward launch")) return WR_BAD_INPUTS;
+    if (!cuda_ok(d, wr::diff::launch_diff_backward(a, d->sms, d->stream), "k_diff_backward launch"))
+        return WR_BAD_INPUTS;
     wr::diff::k_diff_reduce<<<1, 64, 0, d->stream>>>(d->mbar, d->mult, d->n, d_pbar);
     if (!cuda_ok(d, cudaStreamSynchronize(d->stream), "k_diff_backward")) return WR_BAD_INPUTS;
     return WR_SUCCESS;

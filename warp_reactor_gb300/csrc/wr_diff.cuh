@@ -17,7 +17,7 @@
 // xn[0..13] and T.  With the schedule of a plain run and p == 0 the forward map
 // reproduces that run bit for bit.
 //
-// Kernels (one thread per cell; cells are independent once the schedule is given):
+// Kernels (one warp per cell; cells are independent once the schedule is given):
 //   k_diff_forward   the cell's whole schedule with the reference controller
 //                    (RODAS::integrate, :7205-7347); stores per outer step the
 //                    cell's state at the start of the step (18 doubles,
@@ -44,13 +44,8 @@
 //   stage  [n][32][271] LU, pivots and stage vectors of those steps (backward scratch)
 //   mbar   [n][P]       per-cell multiplier adjoints
 //
-// Source files: wr_diff.cu (forward kernel, C ABI), wr_diff_bwd.cu (adjoint
-// kernel), wr_diff_net.cu (network RHS/Jacobian and RHS vector-Jacobian product),
-// wr_diff_jvjp0.cu / wr_diff_jvjp1.cu (Jacobian vector-Jacobian product in
-// chunks).  They are compiled as relocatable device code and device-linked: the
-// generated derivative code is tens of thousands of statements, and one
-// translation unit of it takes ptxas minutes; split, the pieces compile in
-// parallel.
+// Source files: wr_diff.cu (C ABI), wr_diff_coop.cu (both kernels), gen/coop_adj.py (the
+// network's programs they run).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -62,10 +57,9 @@
 namespace wr {
 namespace diff {
 
-constexpr int NP = 44;        // rate-coefficient multipliers (WR_NUM_RATE_MULT, checked where generated code is included)
+constexpr int NP = 44;        // rate-coefficient multipliers (checked where generated code is included)
 constexpr int kFields = 18;   // xn[14], T, e, rho, driver
 constexpr int kSeg = 32;      // accepted steps between burn checkpoints
-constexpr int kThreads = 32;  // one warp per block: a small grid spreads over all SMs
 // per-step record of the adjoint's segment pass: LU (225), pivots (1), k1, k2, k3
 constexpr int kStageIp = NEQ * NEQ;
 constexpr int kStageK1 = kStageIp + 1;
@@ -74,23 +68,6 @@ constexpr int kStageK3 = kStageK2 + NEQ;
 constexpr int kStage = kStageK3 + NEQ;
 
 using M = PortableMath;
-
-struct MatL {
-    double* a;
-    __device__ __forceinline__ double& operator()(int r, int c) const { return a[r * NEQ + c]; }
-};
-
-struct LocalJSink {
-    double* J;
-    __device__ __forceinline__ void operator()(int r, int c, double v) { J[r * NEQ + c] = v; }
-};
-
-// network routines (wr_diff_net.cu, wr_diff_jvjp1.cu), one out-of-line copy each
-__device__ void net_jac(const double* X, double T, double* J);
-__device__ void net_rhs(const double* X, double T, const double* mult, double* f);
-__device__ void net_rhs_vjp(const double* X, double T, const double* mult, const double* fbar, double* Xbar,
-                            double* Tbar, double* mbar);
-__device__ void net_jac_vjp(const double* X, double T, const double* Jbar, double* Xbar, double* Tbar);
 
 struct Args {
     const wr_collapse_state* cells;
@@ -104,6 +81,7 @@ struct Args {
     double* hbuf;
     double* q;              // [n][15]
     int* status;            // [n]
+    int* queue;             // cells taken by the running kernel
     // backward
     const double* qbar;     // [n][15]
     double* ubar;           // [n][15]
@@ -113,18 +91,8 @@ struct Args {
     double* mbar;           // [n][P]
 };
 
-// forward pieces (wr_diff.cu)
-__device__ void ros2s_stages(const double* y, double h, MatL E, uint64_t ip, const double* mult, double* ak1,
-                             double* ak2, double* ak3, double* ynew, double* work);
-__device__ int factor(const double* J, double h, MatL E, uint64_t& ip);
-// one accepted step of the frozen controller; with st != nullptr it also stores
-// the step's factorised iteration matrix, pivots and stage vectors (kStage doubles)
-__device__ void step_replay(double* y, double h, const double* mult, double* st);
-
-__global__ void k_diff_forward(Args a);
-__global__ void k_diff_backward(Args a);
-__global__ void k_diff_mult(const double* logm, double* mult);
-__global__ void k_diff_reduce(const double* mbar, const double* mult, int n, double* pbar);
+cudaError_t launch_diff_forward(Args a, int sms, cudaStream_t stream);
+cudaError_t launch_diff_backward(Args a, int sms, cudaStream_t stream);
 
 struct CellS {
     double xn[NS], T, e, rho, driver;

@@ -23,6 +23,9 @@ not rescaled: the integrator keeps the reference's Jacobian of the unscaled netw
 (at ``mult == 1`` the two coincide); the discrete adjoint differentiates exactly
 the map that is computed.
 
+The GPU kernels run the same derivatives as vector programs (``coop_adj.py``, operation
+for operation in this code's order); the code emitted here is the CPU oracle's.
+
 All emitted code is straight-line C++ over a math policy ``M`` (``exp``, ``log``,
 ``sqrt``, ``fabs``, ``div``), like the network itself.
 """

@@ -95,6 +95,7 @@ from __future__ import annotations
 
 import collections
 import concurrent.futures
+import hashlib
 import math
 import os
 import random
@@ -106,6 +107,9 @@ from . import ir_io
 
 # main classes
 C_NONE, C_FMA, C_EXP, C_LOG, C_SQRT, C_DIV = 0, 1, 2, 3, 4, 5
+# of derivative programs (coop_adj.py): guarded g * x and g / x, which are 0 where g is
+# zero, whatever x holds
+C_GMUL, C_GDIV = 6, 7
 # integer ops: every copy / and / or / not / select is one select A ? B : C (with
 # the boolean constants 0 and 1 as operands); comparisons A <= B, A < B; a sign
 # operation on A (flip the sign bit, or clear it)
@@ -114,14 +118,14 @@ I_SEL, I_LE, I_LT, I_SGN = 0, 1, 2, 3
 SPECIAL_OPS = ("le", "lt", "sneg", "sabs")  # integer nodes that are not selects
 FMA_OPS = ("add", "sub", "mul")
 MAIN_CLASS = {"add": C_FMA, "sub": C_FMA, "mul": C_FMA, "exp": C_EXP, "cexp": C_EXP, "log": C_LOG,
-              "clog": C_LOG, "sqrt": C_SQRT, "csqrt": C_SQRT, "div": C_DIV}
+              "clog": C_LOG, "sqrt": C_SQRT, "csqrt": C_SQRT, "div": C_DIV, "gmul": C_GMUL, "gdiv": C_GDIV}
 INT_OP = {"le": I_LE, "lt": I_LT, "and": I_SEL, "or": I_SEL, "not": I_SEL, "sel": I_SEL, "sneg": I_SGN,
           "sabs": I_SGN}
 # FP64 issue slots of one step of each class (measured call throughput of CUDA's
 # exp/log/sqrt on GB300; division runs on the integer pipe)
-STEP_COST = {C_FMA: 1.0, C_EXP: 19.0, C_LOG: 29.0, C_SQRT: 9.0, C_DIV: 0.5}
+STEP_COST = {C_FMA: 1.0, C_EXP: 19.0, C_LOG: 29.0, C_SQRT: 9.0, C_DIV: 0.5, C_GMUL: 1.0, C_GDIV: 0.5}
 # latency weights for the critical-path priority
-LATENCY = {C_FMA: 1.0, C_EXP: 3.0, C_LOG: 3.0, C_SQRT: 2.0, C_DIV: 2.0, "int": 1.0}
+LATENCY = {C_FMA: 1.0, C_EXP: 3.0, C_LOG: 3.0, C_SQRT: 2.0, C_DIV: 2.0, C_GMUL: 2.0, C_GDIV: 3.0, "int": 1.0}
 
 E_SLOTS = 225
 Y_BASE = 225
@@ -150,7 +154,8 @@ ABS = SIGN - 1
 # leaves of a program: inputs, constants, and transcendentals of constants
 # ("dconst": evaluated once per launch on the device, with the kernel's own
 # exp/log/sqrt, into reserved slots)
-LEAF = ("in", "const", "dconst")
+# ("fix", key): a slot the kernel fills before the program runs (``res`` maps the key)
+LEAF = ("in", "const", "dconst", "fix")
 TRANSCENDENTAL = {"exp": C_EXP, "cexp": C_EXP, "log": C_LOG, "clog": C_LOG, "sqrt": C_SQRT, "csqrt": C_SQRT}
 
 FLOOR = 1.0e-100  # reproducer.cpp:231
@@ -254,7 +259,7 @@ def specialize(P: Program, out: dict, lo: float, hi: float) -> tuple:
         v = abs(v) if ab else v
         return -v if neg else v
 
-    ends = {T: (math.nextafter(lo, math.inf), hi)}
+    ends = {T: (math.nextafter(lo, math.inf), hi) if lo > -math.inf else None}
 
     def interval(x):
         if x not in ends:
@@ -288,7 +293,7 @@ def specialize(P: Program, out: dict, lo: float, hi: float) -> tuple:
         if op == "const":
             m[x] = Q.const_bits(a[0])
             continue
-        if op == "in":
+        if op in ("in", "fix"):
             m[x] = node(op, *a)
             continue
         b = [m[y] for y in a]
@@ -307,6 +312,15 @@ def specialize(P: Program, out: dict, lo: float, hi: float) -> tuple:
             r = false if b[0] == true else true if b[0] == false else None
         elif op == "sel":
             r = b[1] if b[0] == true or b[1] == b[2] else b[2] if b[0] == false else None
+        elif op in ("neg", "abs") and Q.nodes[b[0]][0] == "const":
+            bits = Q.nodes[b[0]][1][0]
+            r = Q.const_bits(bits ^ SIGN if op == "neg" else bits & ABS)
+        elif op in ("gmul", "gdiv") and b[0] == false:  # (false is +0.0)
+            r = false
+        elif op in FMA_OPS:
+            v = [struct.unpack("<d", struct.pack("<Q", Q.nodes[y][1][0]))[0] for y in b if Q.nodes[y][0] == "const"]
+            if len(v) == 2:  # literals are binary64: the same rounding here
+                r = Q.const(v[0] * v[1] if op == "mul" else v[0] + v[1] if op == "add" else v[0] - v[1])
         m[x] = node(op, *b) if r is None else r
     new = {"rhs": [m[x] for x in out["rhs"]], "T": m[T]}
     if "jac" in out:
@@ -447,6 +461,10 @@ def lower(P: Program) -> None:
         op, a = P.nodes[x]
         if op in FMA_OPS or op in INT_OP:
             P.nodes[x] = (op, tuple(plain(y) for y in a))
+        elif op == "gmul":
+            P.nodes[x] = (op, tuple(plain(y) for y in a))
+        elif op == "gdiv" and resolve(P, a[1])[2]:
+            P.nodes[x] = (op, (a[0], plain(a[1])))
 
 
 def live_nodes(P: Program, roots, leaves=False) -> list:
@@ -534,7 +552,8 @@ def list_schedule(comp, args, users, kind, prio, G, limit=None, hold=None, fill=
     steps = []
     left = len(comp)
     live = 0
-    mains = (C_FMA, C_EXP, C_LOG, C_SQRT, C_DIV)
+    mains = (C_FMA, C_EXP, C_LOG, C_SQRT, C_DIV, C_GMUL, C_GDIV)
+    cheap_classes = (C_FMA, C_DIV, C_GMUL, C_GDIV)
 
     def key(x):
         if limit is not None and live >= limit:
@@ -554,12 +573,12 @@ def list_schedule(comp, args, users, kind, prio, G, limit=None, hold=None, fill=
         cls, take = C_NONE, []
         # a thin step now and the rest of its nodes one step later would take two FP64
         # issue slots: wait for them
-        wait = (cand and later.get(len(steps) + 1) and len(ready[C_FMA]) < fill and
+        wait = (cand and later.get(len(steps) + 1) and len(ready[C_FMA]) < fill and len(ready[C_GMUL]) < fill and
                 all(len(ready[c]) < G for c in cand) and not (steps and steps[-1][0] == C_NONE))
         if cand and not wait:
             full = [c for c in cand if len(ready[c]) >= G]
             pool = full if full else cand
-            cheap = [c for c in cand if c in (C_FMA, C_DIV)]
+            cheap = [c for c in cand if c in cheap_classes]
             if hold is not None and not full and cheap:
                 lead = max(top(c) for c in cheap)
                 hc = hold if isinstance(hold, dict) else {c: hold for c in mains}
@@ -650,7 +669,7 @@ def schedule(P: Program, out: dict, G: int, jac: bool, limit=None, first_scratch
     assert len(order) == len(comp), "the program has a cycle"
     lat_t, hold, seed, amp, fill = (tuple(tune) + (1e-3, 0)[len(tune) - 3:])[:5] if tune else (LATENCY[C_EXP], None, 0, 0.0, 0)
     lat = dict(LATENCY)
-    lat.update({C_FMA: float(MAIN_DELAY), C_DIV: 3.0, C_EXP: lat_t, C_LOG: lat_t, C_SQRT: max(1.0, lat_t - 1.0)})
+    lat.update({C_FMA: float(MAIN_DELAY), C_GMUL: float(MAIN_DELAY), C_DIV: 3.0, C_EXP: lat_t, C_LOG: lat_t, C_SQRT: max(1.0, lat_t - 1.0)})
     rng = random.Random(seed)
     prio = {}
     for x in reversed(order):
@@ -956,7 +975,8 @@ def encode(P: Program, sch: Schedule, res: dict) -> list:
 
     def slot_of(b):
         op = P.nodes[b][0]
-        return res[P.nodes[b][1][0]] if op == "const" else res[P.nodes[b][1]] if op == "dconst" else sch.slot[b]
+        return (res[P.nodes[b][1][0]] if op == "const" else res[P.nodes[b][1]] if op in ("dconst", "fix")
+                else sch.slot[b])
 
     def plain(x):  # slot of an operand without modifiers (constants: reserved)
         b, neg, ab = resolve(P, x)
@@ -999,6 +1019,15 @@ def encode(P: Program, sch: Schedule, res: dict) -> list:
                         X, Y, Z, L = ONE, ZERO, plain(a[0]), cbits(a[1]) ^ SIGN
                     else:  # a - b = fma(b, -1, a); K - b reads K from its reserved slot
                         X, Y, Z = plain(a[1]), MONE, plain(a[0])
+                elif op == "gmul":
+                    X, Z = plain(a[0]), MZERO
+                    Y, L = (ZERO, cbits(a[1])) if const(a[1]) else (plain(a[1]), 0)
+                elif op == "gdiv":
+                    (X, xf) = arg(a[0])
+                    if const(a[1]):
+                        Y, L = ZERO, cbits(a[1])
+                    else:
+                        Y, yf = arg(a[1])
                 elif op == "div":
                     num, den = a
                     if const(num):  # K / b: V[Y] ^ L = K, divided by V[X] = b
@@ -1075,11 +1104,11 @@ def device_words(pr: dict, nv: int) -> tuple:
             xf, yf, fl = x & 7, y & 7, 0
             if cls == C_NONE:
                 d = sink >> 48
-            elif cls == C_DIV:
+            elif cls in (C_DIV, C_GDIV):
                 assert not yf & FL_ABS, "absolute value on the literal side of a division"
                 fl = (DV_NEG if xf & FL_NEG else 0) | (DV_ABS if xf & FL_ABS else 0) | (DV_SWAP if yf & FL_SWAP else 0)
                 lit ^= SIGN if yf & FL_NEG else 0
-            elif cls != C_FMA:
+            elif cls not in (C_FMA, C_GMUL):
                 if yf & FL_ABS:
                     fl = DV_ABS | (DV_NEG if yf & FL_NEG else 0)
                 else:
@@ -1350,28 +1379,48 @@ GEN_DIR = os.path.join(os.path.dirname(HERE), "csrc", "generated")
 LANES_PER_CELL = (8, 16, 32)
 
 
+def generator_digest(ir_path: str = ir_io.DEFAULT_PATH) -> str:
+    """Digest of everything the headers are made from."""
+    h = hashlib.sha256()
+    for f in ("coop.py", "coop_adj.py", "adjoint.py", "emit.py", "ir_io.py", "network_dag.py"):
+        with open(os.path.join(HERE, f), "rb") as src:
+            h.update(src.read())
+    with open(ir_path, "rb") as src:
+        h.update(src.read())
+    return h.hexdigest()
+
+
 def _emit_one(G: int, out_dir: str, ir_path: str) -> str:
     from .build_network import _write_if_changed
     path = os.path.join(out_dir, f"coop_prog_g{G}.h")
     gen = generate(G, ir_io.load(ir_path), regimes=REGIMES if G in REGIME_LANES else ())
-    _write_if_changed(path, emit_header(G, gen, ir_io.digest(ir_path)))
+    _write_if_changed(path, f"// generator {generator_digest(ir_path)}\n" + emit_header(G, gen, ir_io.digest(ir_path)))
     return path
 
 
 def emit_all(out_dir: str = GEN_DIR, ir_path: str = ir_io.DEFAULT_PATH) -> list:
-    """The headers of every lane width, one process each (seconds of scheduling).
-    Nothing is rewritten when they are newer than the generator and network.ir."""
-    paths = [os.path.join(out_dir, f"coop_prog_g{G}.h") for G in LANES_PER_CELL]
-    deps = [os.path.join(HERE, f) for f in ("coop.py", "ir_io.py", "network_dag.py")] + [ir_path]
-    if all(os.path.exists(p) and os.path.getmtime(p) >= max(map(os.path.getmtime, deps)) for p in paths):
-        return paths
-    with concurrent.futures.ThreadPoolExecutor(len(LANES_PER_CELL)) as ex:
-        cmd = "import sys; from warp_reactor_gb300.gen import coop; coop._emit_one(int(sys.argv[1]), *sys.argv[2:])"
-        jobs = [ex.submit(subprocess.run, [sys.executable, "-c", cmd, str(G), out_dir, ir_path], check=True,
-                          cwd=os.path.dirname(os.path.dirname(HERE))) for G in LANES_PER_CELL]
-        for j in jobs:
-            j.result()
-    return paths
+    """The headers of every lane width and of the differentiation form, one process
+    each (seconds of scheduling); a header whose first line names the present
+    generator is kept."""
+    jobs = {f"coop_prog_g{G}.h": f"coop._emit_one({G}, *sys.argv[1:])" for G in LANES_PER_CELL}
+    jobs["coop_diff.h"] = "coop_adj.emit(*sys.argv[1:])"
+    want = f"// generator {generator_digest(ir_path)}"
+    paths = {f: os.path.join(out_dir, f) for f in jobs}
+
+    def current(path):
+        if not os.path.exists(path):
+            return False
+        with open(path) as src:
+            return src.readline().strip() == want
+
+    todo = [f for f in jobs if not current(paths[f])]
+    root = os.path.dirname(os.path.dirname(HERE))
+    with concurrent.futures.ThreadPoolExecutor(len(jobs)) as ex:
+        runs = [ex.submit(subprocess.run, [sys.executable, "-c", "import sys; from warp_reactor_gb300.gen import coop, "
+                                           "coop_adj; " + jobs[f], out_dir, ir_path], check=True, cwd=root) for f in todo]
+        for r in runs:
+            r.result()
+    return list(paths.values())
 
 
 if __name__ == "__main__":
