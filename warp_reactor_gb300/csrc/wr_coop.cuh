@@ -99,22 +99,14 @@ __device__ __forceinline__ void sts64(uint32_t addr, uint64_t v) {
 __device__ __forceinline__ uint32_t addr_lo(uint32_t w, uint32_t base) { return __dp2a_lo(w, 0x0001u, base); }
 __device__ __forceinline__ uint32_t addr_hi(uint32_t w, uint32_t base) { return __dp2a_lo(w, 0x0100u, base); }
 
-// IEEE a <= b and a < b on bit patterns: false when either is NaN, -0 == +0
-__device__ __forceinline__ uint64_t ble(uint64_t a, uint64_t b) {
-    const uint64_t ma = a & kAbs, mb = b & kAbs;
-    const bool nan = (ma > kInfBits) | (mb > kInfBits);
-    const bool zero = (ma | mb) == 0;
-    const bool sa = (a >> 63) != 0, sb = (b >> 63) != 0;
-    const bool same = sa ? (ma >= mb) : (ma <= mb);
-    return (!nan && (zero || (sa != sb ? sa : same))) ? 1ULL : 0ULL;
-}
-__device__ __forceinline__ uint64_t blt(uint64_t a, uint64_t b) {
-    const uint64_t ma = a & kAbs, mb = b & kAbs;
-    const bool nan = (ma > kInfBits) | (mb > kInfBits);
-    const bool zero = (ma | mb) == 0;
-    const bool sa = (a >> 63) != 0, sb = (b >> 63) != 0;
-    const bool same = sa ? (ma > mb) : (ma < mb);
-    return (!nan && !zero && (sa != sb ? sa : same)) ? 1ULL : 0ULL;
+// IEEE a <= b (le) or a < b on bit patterns: false when either is NaN, -0 == +0.  a <= b
+// is the negation of b < a; as signed integers, two patterns order like their values
+// unless both are negative.
+__device__ __forceinline__ uint64_t compare(uint64_t a, uint64_t b, bool le) {
+    const int64_t x = static_cast<int64_t>(le ? b : a), y = static_cast<int64_t>(le ? a : b);
+    const bool lt = ((x & y) < 0 ? y < x : x < y) && ((x | y) & static_cast<int64_t>(kAbs)) != 0;
+    const bool nan = (a & kAbs) > kInfBits || (b & kAbs) > kInfBits;
+    return (lt != le) && !nan ? 1ULL : 0ULL;
 }
 
 // Transcendentals are one out-of-line copy each (CUDA's own functions inside for
@@ -147,15 +139,14 @@ __device__ __noinline__ uint64_t slow_step(uint32_t cls, uint64_t x, uint64_t y,
 }
 
 // the integer node of a step: iw = A | B | C | D2
-static __device__ __noinline__ void int_step(uint32_t c, uint64_t iw, uint32_t vb) {
+__device__ __forceinline__ void int_step(uint32_t c, uint64_t iw, uint32_t vb) {
     const uint32_t i0 = static_cast<uint32_t>(iw), i1 = static_cast<uint32_t>(iw >> 32);
     const uint64_t A = lds64(addr_lo(i0, vb)), B = lds64(addr_hi(i0, vb)), C = lds64(addr_lo(i1, vb));
     uint64_t v = A != 0 ? B : C;
     if (c & CTL_SPECIAL) {  // comparisons or sign operations
         const uint32_t d2 = i1 >> 16, iop = d2 & 3u;
-        v = iop == I_LE ? ble(A, B) : v;
-        v = iop == I_LT ? blt(A, B) : v;
-        v = iop == I_SGN ? ((d2 & FL_SABS) ? (A & kAbs) : (A ^ kSign)) : v;
+        const uint64_t s = (d2 & FL_SABS) ? (A & kAbs) : (A ^ kSign);
+        v = iop == I_SEL ? v : iop == I_SGN ? s : compare(A, B, iop == I_LE);
     }
     sts64(addr_hi(i1, vb) & ~7u, v);
 }
@@ -183,8 +174,11 @@ static __device__ __noinline__ void int_step(uint32_t c, uint64_t iw, uint32_t v
 // steps ahead, made every step wait for the L2 latency of the newest one, since the
 // few scoreboards of a warp are shared with the operand loads (Jacobian program at 16
 // lanes, CUDA math, 16 warps in one block: 345 k cycles a run, 264 k in batches; a
-// lone warp 211 k and 173 k).  The tables carry four idle steps past the end.  One
-// out-of-line copy serves every call site: the instruction cache holds one loop.
+// lone warp 211 k and 173 k).  The next four steps' control word is read with them: read
+// at its first use, its constant-cache latency stood in every iteration (a lone warp at 32
+// lanes 97.3 k and 90.9 k).  The integer node is part of the loop (a call per node: 90.9 k
+// and 85.5 k).  The tables carry four idle steps past the end.  One out-of-line copy
+// serves every call site: the instruction cache holds one loop.
 __device__ __forceinline__ ulonglong2 ld_words(const ulonglong2* p) {
     ulonglong2 v;
     asm volatile("ld.global.nc.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p));
@@ -222,6 +216,7 @@ __device__ __noinline__ void run_prog(int which, int gl, uint64_t* V) {
         y = lds64(addr_hi(w0, vb)) ^ l;
         z = lds64(addr_lo(w1, vb));
     };
+    uint32_t c0 = Tab::ctl(ctl0);
     operands(a.e[0], a.l[0]);
     uint64_t res = 0;                         // the last step's main results,
     uint32_t dst = vb + (Tab::kNV - 1) * 8;   // stored while this step's run
@@ -245,7 +240,7 @@ __device__ __noinline__ void run_prog(int which, int gl, uint64_t* V) {
     };
 #pragma unroll 1
     for (int s = 0; s < nsteps; s += 4) {
-        const uint32_t c0 = Tab::ctl(ctl0 + s / 4);
+        const uint32_t cn = Tab::ctl(ctl0 + s / 4 + 1);
         p += 4 * G;
         q += 4 * G;
         b.load(p, q);
@@ -254,6 +249,7 @@ __device__ __noinline__ void run_prog(int which, int gl, uint64_t* V) {
         step(a.e[2], c0 >> 16, a.e[3], a.l[3]);
         step(a.e[3], c0 >> 24, b.e[0], b.l[0]);
         a = b;
+        c0 = cn;
     }
     sts64(dst, res);
     __syncwarp();
@@ -417,8 +413,9 @@ __device__ __forceinline__ void diag_recips(const double* LU, uint64_t (&rY)[K],
 
 // lu_solve<15> (reproducer.cpp:154-181) with x distributed over the group; the
 // back substitution's quotients use the pivots' precomputed reciprocals (the same
-// IEEE quotients as a division).  The next column's factors are loaded while a
-// column's chain (broadcast, quotient, multiply, add) runs.
+// IEEE quotients as a division), inline (a call for each: 32.1 k cycles for a lone cell's
+// three solves, 29.4 k without).  The next column's factors are loaded while a column's
+// chain (broadcast, quotient, multiply, add) runs.
 template <int K>
 struct Vec {
     double v[K];
@@ -470,7 +467,7 @@ __device__ __noinline__ Vec<K> solve_copy(const double* LU, uint64_t ip, uint64_
         for (int t = 0; t < K; ++t) ln[t] = row[t][kn];
         const double dn = LU[kn * NEQ + kn];
         const uint64_t yk = get<G, K>(rY, k);
-        const double q = ddiv_recip(get<G, K>(x, k), d, yk);
+        const double q = wr_div_finish(get<G, K>(x, k), d, yk);
         const double tk = -q;
 #pragma unroll
         for (int t = 0; t < K; ++t) {

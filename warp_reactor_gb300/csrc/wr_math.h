@@ -184,8 +184,11 @@ WR_MHD uint64_t wr_div_recip(double b) {
 // a / b given Y = wr_div_recip(b): the quotient's 54 bits Q = floor(a_m 2^(53+adj) /
 // b_m) from the estimate with Y (Y's error moves it by less than 2^-5, so it is Q or
 // Q - 1), its exact remainder, round to nearest even.  Operands or quotients outside
-// the normal range divide by a / b; one exit for all of them, since a copy of the
-// native division costs the kernels' instruction cache two kilobytes.
+// the normal range divide by a / b, out of line and one exit for all of them: a copy
+// of the native division costs the kernels' instruction cache two kilobytes.
+#if defined(__CUDACC__)
+static __device__ __noinline__ double wr_div_native(double a, double b) { return a / b; }
+#endif
 WR_MHD double wr_div_finish(double a, double b, uint64_t Y) {
     const uint64_t ua = wr_bits(a), ub = wr_bits(b);
     const uint32_t ea = static_cast<uint32_t>(ua >> 52) & 0x7ff;
@@ -209,7 +212,11 @@ WR_MHD double wr_div_finish(double a, double b, uint64_t Y) {
         const uint64_t r = (static_cast<uint64_t>(static_cast<uint32_t>(be)) << 52) + mant + up;
         return wr_from_bits(r | ((ua ^ ub) & 0x8000000000000000ULL));
     }
+#if defined(__CUDA_ARCH__)
+    return wr_div_native(a, b);
+#else
     return a / b;
+#endif
 }
 
 WR_MHD double wr_div_int(double a, double b) { return wr_div_finish(a, b, wr_div_recip(b)); }

@@ -522,7 +522,7 @@ class Schedule:
         self.consts = consts
 
 
-def list_schedule(comp, args, users, kind, prio, G, limit=None, hold=None, fill=0):
+def list_schedule(comp, args, users, kind, prio, G, limit=None, hold=None, fill=0, ifill=0):
     """Steps of width G: each step takes up to G ready nodes of one main class
     (highest priority first; a full step is preferred) and up to G ready integer
     nodes.  ``args``/``users`` give the dependences in the direction scheduled.  A
@@ -535,7 +535,9 @@ def list_schedule(comp, args, users, kind, prio, G, limit=None, hold=None, fill=
     ``hold`` (a number, or one per class; None: no such rule).
 
     ``fill``: with fewer ready FMA nodes than that, and more becoming ready at the next
-    step, a step is left without a main node (never two in a row).
+    step, a step is left without a main node (never two in a row).  ``ifill``: with fewer
+    ready integer nodes than that, none of them as critical as a ready main node, they
+    wait (a step with integer nodes costs six shared accesses more, for one or for G).
 
     ``limit``: once that many computed values are live (computed, with users not
     yet scheduled), ready nodes are taken by their effect on the live set first
@@ -567,9 +569,12 @@ def list_schedule(comp, args, users, kind, prio, G, limit=None, hold=None, fill=
     while left:
         for x in later.pop(len(steps), []):
             ready[kind(x)].append(x)
-        rl = sorted(ready["int"], key=key)
-        riders, ready["int"] = rl[:G], rl[G:]
         cand = [c for c in mains if ready[c]]
+        rl = sorted(ready["int"], key=key)
+        n = G
+        if cand and 0 < len(rl) < ifill and max(prio[x] for x in rl) < max(top(c) for c in cand):
+            n = 0
+        riders, ready["int"] = rl[:n], rl[n:]
         cls, take = C_NONE, []
         # a thin step now and the rest of its nodes one step later would take two FP64
         # issue slots: wait for them
@@ -640,7 +645,7 @@ def schedule(P: Program, out: dict, G: int, jac: bool, limit=None, first_scratch
     ``first_scratch``: the first slot above the reserved constants.  ``tune``:
     (latency weight of exp/log/sqrt, ``hold`` of the list scheduler, seed of a
     random perturbation of the priorities (0: none)[, its amplitude, 1e-3 by
-    default[, ``fill`` of the list scheduler]]) -- the schedule is a heuristic, and these pick among equally valid
+    default[, ``fill``[, ``ifill``] of the list scheduler]]) -- the schedule is a heuristic, and these pick among equally valid
     ones.  ``banked``: (reserved slot map, slot cap) to allocate slots with
     ``allocate_banked`` (G = 16), falling back to the linear scan when it finds
     no room below the cap."""
@@ -667,7 +672,8 @@ def schedule(P: Program, out: dict, G: int, jac: bool, limit=None, first_scratch
             if pend[u] == 0:
                 order.append(u)
     assert len(order) == len(comp), "the program has a cycle"
-    lat_t, hold, seed, amp, fill = (tuple(tune) + (1e-3, 0)[len(tune) - 3:])[:5] if tune else (LATENCY[C_EXP], None, 0, 0.0, 0)
+    lat_t, hold, seed, amp, fill, ifill = ((tuple(tune) + (1e-3, 0, 0)[len(tune) - 3:])[:6] if tune else
+                                           (LATENCY[C_EXP], None, 0, 0.0, 0, 0))
     lat = dict(LATENCY)
     lat.update({C_FMA: float(MAIN_DELAY), C_GMUL: float(MAIN_DELAY), C_DIV: 3.0, C_EXP: lat_t, C_LOG: lat_t, C_SQRT: max(1.0, lat_t - 1.0)})
     rng = random.Random(seed)
@@ -675,7 +681,7 @@ def schedule(P: Program, out: dict, G: int, jac: bool, limit=None, first_scratch
     for x in reversed(order):
         prio[x] = lat[kind(x)] + max((prio[u] for u in users[x]), default=0.0)
         prio[x] += rng.random() * amp if seed else 0.0
-    steps = sink_riders(list_schedule(comp, cargs, users, kind, prio, G, limit, hold, fill), users, kind, G)
+    steps = sink_riders(list_schedule(comp, cargs, users, kind, prio, G, limit, hold, fill, ifill), users, kind, G)
     done_at = {}
     for s, (cls, take, riders) in enumerate(steps):
         for x in take + riders:
@@ -1123,40 +1129,42 @@ def device_words(pr: dict, nv: int) -> tuple:
 # count among limits that do not add FP64 issue slots)
 SCHED_LIMIT = {8: 400, 16: 350, 32: 600}
 # scheduler tuning per G and program: (schedule()'s ``tune``, live-set limit),
-# chosen offline by a seeded random search for the fewest FP64 issue slots of the
-# program whose slot count keeps the block's warps (16 lanes: 16 warps, <= 907
+# chosen offline by a seeded random search for the fewest FP64 issue slots (at 32
+# lanes the fewest cycles of a lone warp, an integer node's 350 included) of the
+# program whose slot count keeps the block's warps (16 lanes: 16 warps, <= 903
 # slots; 8 lanes: 9 warps, <= 807 slots)
 SCHED_TUNE = {
     16: {
-        "jrhs": ((2.0, 8.0, 80444, 0.01, 8), 350),
+        "jrhs": ((4, None, 759535, 0.001, 10, 12), 500),
         "rhs": ((4.0, 8.0, 913542, 0.5, 14), 425),
-        (1, "jrhs"): ((3.0, None, 998460, 0.01, 14), 350),
+        (1, "jrhs"): ((2.0, None, 817964, 0.01, 9, 15), 400),
         (1, "rhs"): ((1.5, {C_EXP: 2.0, C_LOG: 2.0, C_SQRT: 20.0}, 109686, 1.0, 14), 600),
-        (2, "jrhs"): ((4.0, 0.0, 68050, 1.0, 11), 500),
+        (2, "jrhs"): ((3.5, 0.0, 144618, 1.0, 11, 12), 500),
         (2, "rhs"): ((4.5, 8.0, 105236, 0.001, 13), 600),
-        (3, "jrhs"): ((2.0, 1.0, 544639, 0.001, 11), 450),
+        (3, "jrhs"): ((2.5, 0.0, 544639, 0.001, 11, 10), 425),
         (3, "rhs"): ((3.0, {C_EXP: 0.0, C_LOG: 10.0, C_SQRT: 20.0}, 505950, 0.5, 13), 475),
-        (4, "jrhs"): ((3.0, 0.0, 164671, 0.001, 10), 600),
+        (4, "jrhs"): ((3.5, 0.0, 693834, 0.001, 10, 15), 500),
         (4, "rhs"): ((1.0, 8.0, 634925, 0.01, 11), 650),
-        (5, "jrhs"): ((6.5, 1.0, 275871, 0.5, 11), 600),
+        (5, "jrhs"): ((6.5, 1.0, 374939, 0.5, 11, 16), 600),
         (5, "rhs"): ((2.0, {C_EXP: 2.0, C_LOG: 10.0, C_SQRT: 20.0}, 11048, 0.5, 13), 550),
-        (6, "jrhs"): ((8.0, None, 437426, 0.001, 10), 475),
+        (6, "jrhs"): ((8.0, None, 294502, 0.001, 12, 14), 475),
         (6, "rhs"): ((3.5, {C_EXP: 2.0, C_LOG: 30.0, C_SQRT: 5.0}, 6388, 0.5, 12), 450),
     },
     32: {
-        "jrhs": ((1.5, 0.0, 849342, 0.001, 20), 600),
+        "jrhs": ((0.5, 2.0, 11371, 0.5, 10, 14), 700),
         "rhs": ((8.0, {C_EXP: 20.0, C_LOG: 30.0, C_SQRT: 5.0}, 620078, 0.1, 23), 450),
-        (1, "jrhs"): ((5.5, None, 378914, 0.1, 30), 525),
+        (1, "jrhs"): ((4.5, None, 978585, 0.1, 30, 7), 475),
         (1, "rhs"): ((3.5, {C_EXP: 20.0, C_LOG: 30.0, C_SQRT: 5.0}, 499564, 2.0, 21), 600),
-        (2, "jrhs"): ((2.5, 0.0, 16209, 0.001, 19), 600),
+        (2, "jrhs"): ((2, {C_EXP: 10.0, C_LOG: 5.0, C_SQRT: 20.0}, 676014, 0.5, 20, 27), 450),
         (2, "rhs"): ((1.5, 8.0, 723724, 2.0, 23), 550),
-        (3, "jrhs"): ((5.5, 2.0, 789616, 0.5, 30), 500),
+        (3, "jrhs"): ((5.5, 2.0, 781275, 0.5, 30, 7), 500),
         (3, "rhs"): ((4.5, {C_EXP: 20.0, C_LOG: 10.0, C_SQRT: 20.0}, 602532, 2.0, 10), 600),
-        (4, "jrhs"): ((6.0, 5.0, 173831, 0.5, 31), 375),
+        (4, "jrhs"): ((7.0, 5.0, 680814, 0.01, 18, 16), 425),
         (4, "rhs"): ((1.0, {C_EXP: 20.0, C_LOG: 5.0, C_SQRT: 0.0}, 421877, 1.0, 32), 700),
-        (5, "jrhs"): ((4.0, 0.0, 585544, 0.001, 19), 600),
+        (5, "jrhs"): ((4.0, 0.0, 514329, 0.01, 19, 5), 625),
         (5, "rhs"): ((8.0, {C_EXP: 20.0, C_LOG: 30.0, C_SQRT: 5.0}, 845573, 2.0, 24), 450),
         (6, "rhs"): ((7.0, {C_EXP: 20.0, C_LOG: 30.0, C_SQRT: 5.0}, 391120, 1.0, 31), 450),
+        (6, "jrhs"): ((2.5, {C_EXP: 0.0, C_LOG: 30.0, C_SQRT: 0.0}, 672671, 0.01, 18, 30), 450),
     },
     8: {"jrhs": ((1.5, 8.0, 899089, 0.5, 7), 400), "rhs": ((1.5, 8.0, 27320, 1.0, 2), 650)},
 }
