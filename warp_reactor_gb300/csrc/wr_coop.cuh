@@ -555,6 +555,37 @@ __device__ __forceinline__ void gather_matrix(uint64_t* V, const uint16_t* jac, 
     __syncwarp();
 }
 
+// E and the RHS of a state, kept in the lanes' local memory for the attempts that
+// retry it with another step size (shared memory has no room for a second matrix at
+// 16 lanes and 16 warps).  A collapse of one cell rejects 27 % of its attempts, one of
+// 64^3 cells 14 %, and the Jacobian program is a third of an attempt: the collapse of one
+// cell 219 -> 198 ms, a step of 16^3 cells 22.3 -> 20.0 ms, of 64^3 234 -> 221 ms.
+template <int G, int K>
+struct Kept {
+    static constexpr bool kOn = true;
+    static constexpr int kRows = (NEQ * NEQ + G - 1) / G;
+    uint64_t m[kRows];
+    double f[K];
+    __device__ __forceinline__ void save(const uint64_t* V, const double (&rhs)[K], int gl) {
+#pragma unroll 4
+        for (int t = 0; t < kRows; ++t)
+            if (gl + t * G < NEQ * NEQ) m[t] = V[kE + gl + t * G];
+#pragma unroll
+        for (int t = 0; t < K; ++t) f[t] = rhs[t];
+    }
+    __device__ __forceinline__ void restore(uint64_t* V, double (&rhs)[K], int gl) const {
+#pragma unroll 4
+        for (int t = 0; t < kRows; ++t)
+            if (gl + t * G < NEQ * NEQ) V[kE + gl + t * G] = m[t];
+#pragma unroll
+        for (int t = 0; t < K; ++t) rhs[t] = f[t];
+        __syncwarp();
+    }
+};
+struct KeepNothing {  // for a caller that never retries
+    static constexpr bool kOn = false;
+};
+
 // Generated tables of one G, supplied by the translation unit that includes the
 // generated header (one unit per G keeps the large initialisers apart).
 //   Tab::kNV, Tab::kNR, Tab::kNF, Tab::kRegimes, Tab::kAdjoint and device accessors vconst(),
@@ -610,16 +641,23 @@ struct PhaseClock<true> {
 // The stages of one ROS2S attempt (reproducer.cpp:7259-7304) of the warp's cells from y
 // with step h: the factorised iteration matrix in the matrix slots, its pivots, k1, k2
 // and k3.  Returns the factorisation's info (0: regular; the rest means nothing
-// otherwise).
-template <class M, int G, class Tab, int K, class PC>
+// otherwise).  again (the same for the whole warp): each cell's y is the one of its
+// last attempt, whose Jacobian and RHS stand in kept; the program does not run.
+template <class M, int G, class Tab, int K, class PC, class Keep>
 __device__ __forceinline__ int ros2s_stages(uint64_t* V, const double (&y)[K], double h, int& regime, int gl, PC& pc,
-                                            uint64_t& ip, double (&ak1)[K], double (&ak2)[K], double (&w)[K]) {
+                                            bool again, Keep& kept, uint64_t& ip, double (&ak1)[K], double (&ak2)[K],
+                                            double (&w)[K]) {
     using namespace coop;
     double* E = reinterpret_cast<double*>(V + kE);
-    const int jw = evaluate<M, G, Tab, K>(0, y, regime, gl, V);
-    pc.mark(PH_JPROG);
-    load_outputs<G, K>(V, Tab::out(jw), ak1, gl);
-    gather_matrix<G>(V, Tab::jac(jw / 2), gl);
+    if (!Keep::kOn || !again) {
+        const int jw = evaluate<M, G, Tab, K>(0, y, regime, gl, V);
+        pc.mark(PH_JPROG);
+        load_outputs<G, K>(V, Tab::out(jw), ak1, gl);
+        gather_matrix<G>(V, Tab::jac(jw / 2), gl);
+        if constexpr (Keep::kOn) kept.save(V, ak1, gl);
+    } else if constexpr (Keep::kOn) {
+        kept.restore(V, ak1, gl);
+    }
     const double fac = ddiv(1.0, h * kGamma);
 #pragma unroll
     for (int t = 0; t < K; ++t) {
@@ -708,12 +746,12 @@ __device__ __forceinline__ void ros2s_candidate(const double (&y)[K], const doub
 }
 
 // One attempt: candidate state, error norm, and the factorisation's info
-template <class M, int G, class Tab, bool FMAX, int K, class PC>
+template <class M, int G, class Tab, bool FMAX, int K, class PC, class Keep>
 __device__ __forceinline__ int ros2s_attempt(uint64_t* V, const double (&y)[K], double h, int& regime, int gl, PC& pc,
-                                             double (&ynew)[K], double& err) {
+                                             bool again, Keep& kept, double (&ynew)[K], double& err) {
     uint64_t ip;
     double ak1[K], ak2[K], ak3[K];
-    const int info = ros2s_stages<M, G, Tab, K>(V, y, h, regime, gl, pc, ip, ak1, ak2, ak3);
+    const int info = ros2s_stages<M, G, Tab, K>(V, y, h, regime, gl, pc, again, kept, ip, ak1, ak2, ak3);
     ros2s_candidate<G, FMAX, K>(y, ak1, ak2, ak3, gl, ynew, err);
     return info;
 }
@@ -744,6 +782,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
     bool drained = false;  // it has seen the queue's end
     int regime = 0;        // the temperature regime of its last evaluation
     double y[K];
+    Kept<G, K> kept;
 #pragma unroll
     for (int t = 0; t < K; ++t) y[t] = 0.0;
 
@@ -845,11 +884,14 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
         pc.mark(PH_QUEUE);
         pc.attempt();
 
+        // a rejected attempt is retried from the same state: where no cell of the warp is
+        // at a new one, the Jacobian and the RHS of the last attempt stand
+        const bool again = !__any_sync(kWarp, have && L.fresh);
         if (L.fresh) L.n_jac += 1;
         L.fresh = false;
         const double h = L.h;
         double ynew[K], err;
-        const int info = ros2s_attempt<M, G, Tab, false, K>(V, y, h, regime, gl, pc, ynew, err);
+        const int info = ros2s_attempt<M, G, Tab, false, K>(V, y, h, regime, gl, pc, again, kept, ynew, err);
         // step-size controller, reproducer.cpp:7308-7344
         const double raw_fac = ddiv(StepMath<M>::cbrt(err), kSafe);
         const double fac_step = smax(1.0 / kFacMax, smin(1.0 / kFacMin, raw_fac));

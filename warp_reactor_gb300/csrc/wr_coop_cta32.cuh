@@ -176,10 +176,12 @@ __global__ void __launch_bounds__(kTileCells / CL * G, 1) k_advance_cta32(DevSta
             if (warp == 0) next_trial();
             __syncthreads();
             int set = 0;
+            bool again = false;  // the last trial was not accepted: the same states
+            Kept<G, K> kept;
             while (tc.run) {
                 double ynew[K], err = 0.0;
                 int info = 0;
-                if (holders) info = ros2s_attempt<M, G, Tab, true, K>(V, y, tc.h, regime, gl, pc, ynew, err);
+                if (holders) info = ros2s_attempt<M, G, Tab, true, K>(V, y, tc.h, regime, gl, pc, again, kept, ynew, err);
                 if (gl == 0) tc.err[set][mine] = !have ? 0.0 : info != 0 ? -1.0 : isfinite(err) ? err : DBL_MAX;
                 tile_sync();
                 if (warp == 0) {
@@ -235,6 +237,7 @@ __global__ void __launch_bounds__(kTileCells / CL * G, 1) k_advance_cta32(DevSta
 #pragma unroll
                     for (int t = 0; t < K; ++t) y[t] = ynew[t];
                 }
+                again = tc.accept == 0;
                 set ^= 1;
             }
 

@@ -109,8 +109,10 @@ __device__ __noinline__ int burn_record(uint64_t* V, double& yl, double tout, do
     double hacc = 0.0, erracc = 1.0, x = 0.0;
     *count = 0;
     PhaseClock<false> pc;
+    coop::Kept<G, 1> kept;
 #pragma unroll 1
     for (;;) {
+        const bool again = !fresh;  // the same state as the last attempt's
         if (fresh) {
             if (n_step > kMaxSteps) return WR_TOO_MANY_STEPS;
             if (0.1 * ::fabs(h) <= ::fabs(x) * kUround) return WR_DT_UNDERFLOW;
@@ -124,7 +126,7 @@ __device__ __noinline__ int burn_record(uint64_t* V, double& yl, double tout, do
         const double y[1] = {yl};
         double k1[1], k2[1], k3[1], ynew[1], err;
         uint64_t ip;
-        const int info = ros2s_stages<CM, G, Tab, 1>(V, y, h, regime, lane, pc, ip, k1, k2, k3);
+        const int info = ros2s_stages<CM, G, Tab, 1>(V, y, h, regime, lane, pc, again, kept, ip, k1, k2, k3);
         if (info != 0) {
             nsing += 1;
             if (nsing >= 5) return WR_LU_DECOMPOSITION_ERROR;
@@ -320,7 +322,7 @@ __device__ __noinline__ double solve_t_coop(const double* LU, uint64_t ip, uint6
     for (int k = 0; k < NEQ; ++k) {
         const double u = lane < NEQ ? LU[k * NEQ + lane] : 0.0;
         const double v[1] = {xx[0] - t};
-        const double q = ddiv_recip(get<G, 1>(v, k), LU[k * NEQ + k], get<G, 1>(yy, k));
+        const double q = wr_div_finish(get<G, 1>(v, k), LU[k * NEQ + k], get<G, 1>(yy, k));
         if (lane == k) xx[0] = q;
         if (lane > k) t += u * q;
     }
@@ -382,7 +384,8 @@ __device__ __noinline__ double step_replay(uint64_t* V, double yl, double h, dou
     double k1[1], k2[1], k3[1];
     uint64_t ip;
     PhaseClock<false> pc;
-    ros2s_stages<CM, G, Tab, 1>(V, y, h, regime, lane, pc, ip, k1, k2, k3);
+    coop::KeepNothing none;
+    ros2s_stages<CM, G, Tab, 1>(V, y, h, regime, lane, pc, false, none, ip, k1, k2, k3);
     if (st != nullptr) {
         for (int k = lane; k < NEQ * NEQ; k += G) st[k] = coop::dbl(V[coop::kE + k]);
         if (lane == 0) st[kStageIp] = __longlong_as_double(static_cast<long long>(ip));
