@@ -24,9 +24,11 @@
 //    (RODAS::integrate, :7205-7347) run per component on the lanes; scalars are
 //    replicated in every lane of the group.
 //
-// A rejected attempt recomputes the Jacobian at the same state: the values are
-// identical (same operations on the same operands), and the warp stays in one
-// instruction stream; the Jacobian counter follows the reference's rule.  Every
+// A rejected attempt is retried from the same state: where every cell of the warp
+// retries, the Jacobian and RHS of the attempt before are used again (Kept); where one
+// is at a new state, the program runs for all of them and gives the retrying ones the
+// same values (same operations on the same operands), so the warp stays in one
+// instruction stream.  The Jacobian counter follows the reference's rule.  Every
 // value is the same binary64 operation on the same operands as in the reference
 // and the CPU oracle, so results are bit-identical.
 //

@@ -30,9 +30,10 @@ constexpr int kDefaultVariant = 6;   // 16 lanes per cell: the most cells per se
 constexpr int kLatencyVariant = 7;   // 32 lanes per cell: the shortest attempt
 // Cells per SM up to which a context takes 32 lanes per cell.  A block holds 16 cells
 // at 32 lanes and 32 at 16: while every cell has its warp at once, an outer step lasts
-// as long as its longest burn, and a 32-lane attempt is shorter (one outer step of 512
-// cells on GB300: 2.35 ms at 32 lanes, 3.24 ms at 16); beyond that the 16-lane shape's
-// rate decides (20,011 cells: 18.3 ms at 32 lanes, 13.3 ms at 16).
+// as long as its longest burn, and a 32-lane attempt is shorter (one outer step on GB300,
+// CUDA math: 512 cells 2.01 ms at 32 lanes, 2.24 ms at 16; 2,432 cells, 16 per SM, 2.52
+// and 3.21 ms); beyond that the 16-lane shape's rate decides (3,000 cells 3.43 and 3.34 ms,
+// 20,011 cells 16.3 and 12.4 ms).
 constexpr int kLatencyCellsPerSm = 16;
 struct AdvanceShape {
     int threads;    // lane-per-cell shapes (0 for the cooperative advance)

@@ -1169,8 +1169,9 @@ SCHED_TUNE = {
     8: {"jrhs": ((1.5, 8.0, 899089, 0.5, 7), 400), "rhs": ((1.5, 8.0, 27320, 1.0, 2), 650)},
 }
 # shared memory of one block (227 KiB) and the warps per block the slot arrays
-# allow, at most 16: at 16 lanes per cell (728 slots) 16 warps ran a 64^3 collapse
-# in 32.5 s on GB300, 17 warps in 34.3 s and 19 warps (register-limited) in 33.3 s
+# allow, at most 16 (the kernels take 128 registers per thread): with an earlier program
+# layout of 728 slots, 16 warps ran a 64^3 collapse in 32.5 s on GB300, 17 warps in
+# 34.3 s and 19 warps in 33.3 s
 SMEM_BLOCK = 232448
 MAX_WARPS = 16
 # lane widths whose slots are allocated bank by bank (allocate_banked)
