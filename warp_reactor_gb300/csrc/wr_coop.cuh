@@ -758,6 +758,31 @@ __device__ __forceinline__ int ros2s_attempt(uint64_t* V, const double (&y)[K], 
     return info;
 }
 
+// The controller's next step sizes (reproducer.cpp:7308-7327) after a step h with error
+// norm err: hnew from err alone, hgus with the Gustafsson factor.  Their two chains
+// (quotient, cube root, quotient, limits, quotient) run side by side, hnew's in the even
+// lanes and hgus's in the odd ones: one cube root and three quotients of latency instead
+// of two and five (a step of 20,011 cells in portable math 20.1 -> 19.8 ms, the structured
+// policy on 1,000 cells 89.2 -> 88.2 ms).  FMAX: limits by fmax and fmin (the structured
+// policy).
+template <int G, bool FMAX, class Cbrt>
+__device__ __forceinline__ void step_sizes(double err, double erracc, double hacc, double h, int gl, Cbrt cbrt,
+                                           double& hnew, double& hgus) {
+    using coop::kWarp;
+    const bool odd = (gl & 1) != 0;
+    const double q = ddiv(odd ? hacc : err * err, odd ? h : erracc);
+    const double e2 = __shfl_sync(kWarp, q, 0, G), ratio = __shfl_sync(kWarp, q, 1, G);
+    const double c = cbrt(odd ? e2 : err);
+    const double raw = ddiv(odd ? ratio * c : c, kSafe);
+    const double f = FMAX ? ::fmax(1.0 / kFacMax, ::fmin(1.0 / kFacMin, raw))
+                          : smax(1.0 / kFacMax, smin(1.0 / kFacMin, raw));
+    const double fs = __shfl_sync(kWarp, f, 0, G), fg = __shfl_sync(kWarp, f, 1, G);
+    const double both = FMAX ? ::fmax(fs, fg) : smax(fs, fg);
+    const double hn = ddiv(h, odd ? both : fs);
+    hnew = __shfl_sync(kWarp, hn, 0, G);
+    hgus = __shfl_sync(kWarp, hn, 1, G);
+}
+
 // The cooperative burn: persistent blocks of W warps, G lanes per cell, each group
 // taking cells from the work queue until it is empty.  PH: the phase-counting
 // instantiation (phases: its 16 counters).
@@ -895,9 +920,8 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
         double ynew[K], err;
         const int info = ros2s_attempt<M, G, Tab, false, K>(V, y, h, regime, gl, pc, again, kept, ynew, err);
         // step-size controller, reproducer.cpp:7308-7344
-        const double raw_fac = ddiv(StepMath<M>::cbrt(err), kSafe);
-        const double fac_step = smax(1.0 / kFacMax, smin(1.0 / kFacMin, raw_fac));
-        double hnew = ddiv(h, fac_step);
+        double hnew, hgus;
+        step_sizes<G, false>(err, L.erracc, L.hacc, h, gl, StepMath<M>::cbrt, hnew, hgus);
         int code = 0;  // a failure that ends the cell's burn
         if (info != 0) {  // singular: the attempt counts for nothing (reproducer.cpp:7268-7277)
             L.nsing += 1;
@@ -912,11 +936,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
             L.n_decomp += 1;
             L.n_step += 1;
             L.n_accept += 1;
-            if (L.n_accept > 1) {
-                const double facgus = smax(1.0 / kFacMax,
-                    smin(1.0 / kFacMin, ddiv(ddiv(L.hacc, h) * StepMath<M>::cbrt(ddiv(err * err, L.erracc)), kSafe)));
-                hnew = ddiv(h, smax(fac_step, facgus));
-            }
+            if (L.n_accept > 1) hnew = hgus;
             L.hacc = h;
             L.erracc = smax(1.e-2, err);
 #pragma unroll

@@ -18,7 +18,7 @@
 // anything else.  A tile's trials are serial, so with few tiles the time is a trial's
 // latency: 32 cells on one SM share its FP64 pipes, 8 cells on each of four SMs at 32
 // lanes per cell run a trial in half the time (the choice is cta32_shape's).  Measured
-// on GB300, 1,000 cells over the last eight outer steps of a collapse: 89 ms; one lane
+// on GB300, 1,000 cells over the last eight outer steps of a collapse: 88 ms; one lane
 // per cell and one warp per tile, as this kernel was before, 1,159 ms.
 #pragma once
 
@@ -202,19 +202,12 @@ __global__ void __launch_bounds__(kTileCells / CL * G, 1) k_advance_cta32(DevSta
                         for (int off = 16; off > 0; off >>= 1) ev = ::fmax(ev, __shfl_xor_sync(kWarp, ev, off));
                         const double err_tile = ev;
                         ++n_step;
-                        const double fac_step =
-                            ::fmax(1.0 / kFacMax, ::fmin(1.0 / kFacMin, ddiv(cbrt_nonnegative<M>(err_tile), kSafe)));
-                        double hnew = ddiv(h, fac_step);
+                        double hnew, hgus;
+                        step_sizes<32, true>(err_tile, erracc, hacc, h, lane, cbrt_nonnegative<M>, hnew, hgus);
                         accept = err_tile <= 1.0;
                         if (accept) {
                             ++n_accept;
-                            if (n_accept > 1) {
-                                const double facgus = ::fmax(1.0 / kFacMax,
-                                    ::fmin(1.0 / kFacMin,
-                                           ddiv(ddiv(hacc, h) * cbrt_nonnegative<M>(ddiv(err_tile * err_tile, erracc)),
-                                                kSafe)));
-                                hnew = ddiv(h, ::fmax(fac_step, facgus));
-                            }
+                            if (n_accept > 1) hnew = hgus;
                             hacc = h;
                             erracc = ::fmax(1.0e-2, err_tile);
                             x = final_trial ? dt_grid : x + h;

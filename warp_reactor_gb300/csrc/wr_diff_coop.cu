@@ -137,17 +137,11 @@ __device__ __noinline__ int burn_record(uint64_t* V, double& yl, double tout, do
         }
         ros2s_candidate<G, false, 1>(y, k1, k2, k3, lane, ynew, err);
         n_step += 1;
-        const double raw_fac = ddiv(coop::StepMath<CM>::cbrt(err), kSafe);
-        const double fac_step = smax(1.0 / kFacMax, smin(1.0 / kFacMin, raw_fac));
-        double hnew = ddiv(h, fac_step);
+        double hnew, hgus;
+        step_sizes<G, false>(err, erracc, hacc, h, lane, coop::StepMath<CM>::cbrt, hnew, hgus);
         if (err <= 1.0) {
             n_accept += 1;
-            if (n_accept > 1) {
-                const double facgus = smax(1.0 / kFacMax,
-                    smin(1.0 / kFacMin,
-                         ddiv(ddiv(hacc, h) * coop::StepMath<CM>::cbrt(ddiv(err * err, erracc)), kSafe)));
-                hnew = ddiv(h, smax(fac_step, facgus));
-            }
+            if (n_accept > 1) hnew = hgus;
             hacc = h;
             erracc = smax(1.e-2, err);
             if (*count >= cap_left) return WR_TOO_MANY_STEPS;
