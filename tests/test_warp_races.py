@@ -1,0 +1,82 @@
+"""The cooperative kernels' device code on the CPU, one thread per lane, under
+ThreadSanitizer (warp_threads/warp_threads.h): lanes that share the slot array are ordered
+by __syncwarp alone, so an access that relies on the warp's lanes staying together is
+reported, whatever order they ran in; and the results equal the CPU oracle's bit for bit."""
+import os
+import re
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "warp_threads")
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "warp_reactor_gb300", "csrc")
+
+# the PTX accesses of wr_coop.cuh, in C++
+PTX = {
+    'asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(addr));': "v = slots[addr / 8];",
+    'asm volatile("st.shared.b64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");': "warp::store(slots, addr, v);",
+    'asm volatile("ld.global.nc.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p));': "v = *p;",
+    'asm volatile("ld.global.nc.u64 %0, [%1];" : "=l"(v) : "l"(p));': "v = *p;",
+}
+
+
+def compile_program(tmp, name, parts, flags=()):
+    """``name``.cpp with the device code ``parts`` as device_code.h, under the sanitizer."""
+    src = open(os.path.join(CSRC, "wr_coop.cuh")).read()
+    for asm, cxx in PTX.items():
+        assert src.count(asm) == 1, asm
+        src = src.replace(asm, cxx)
+    assert "asm" not in src
+    (tmp / "wr_coop.cuh").write_text(src)
+    (tmp / "cuda_runtime.h").write_text("#pragma once\nusing cudaError_t = int;\nusing cudaStream_t = void*;\n")
+    (tmp / "device_code.h").write_text(parts)
+    exe = str(tmp / name)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-g", "-fsanitize=thread", "-ffp-contract=off", "-fno-inline-small-functions",
+                    "-Wno-unknown-pragmas", "-I", str(tmp), "-I", HERE, "-I", CSRC, *flags,
+                    os.path.join(HERE, name + ".cpp"), "-o", exe, "-pthread"], check=True)
+    return exe
+
+
+def run_program(exe, *args):
+    r = subprocess.run([exe, *map(str, args)], capture_output=True, text=True, timeout=600,
+                       env={**os.environ, "TSAN_OPTIONS": "halt_on_error=0 exitcode=66"})
+    if "unexpected memory mapping" in r.stderr:
+        pytest.skip("ThreadSanitizer cannot map its shadow here")
+    races = sorted(set(re.findall(r"SUMMARY: ThreadSanitizer: data race (.*)", r.stderr)))
+    assert not races, "\n".join(races[:20])
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.fixture(scope="module", params=[8, 16, 32])
+def advance(request, built, tmp_path_factory):
+    G = request.param
+    unit = open(os.path.join(CSRC, "wr_adv_coop.cuh")).read()
+    tables = unit[unit.index("namespace cp ="):unit.index("static_assert(coop::kRes")].replace(
+        "WR_CAT(coop, WR_COOP_G)", f"coop{G}")
+    parts = f'#include "generated/coop_prog_g{G}.h"\n#include "wr_coop.cuh"\nnamespace wr {{\n{tables}\n}}\n'
+    return compile_program(tmp_path_factory.mktemp(f"advance{G}"), "advance", parts)
+
+
+def burn(advance, tmp, oracle, wr, cells, dt):
+    rec = np.zeros((len(cells), 16))
+    rec[:, :14], rec[:, 14], rec[:, 15] = cells["xn"], cells["T"], dt
+    (tmp / "in").write_bytes(rec.tobytes())
+    run_program(advance, tmp / "in", tmp / "out")
+    got = np.frombuffer((tmp / "out").read_bytes()).reshape(-1, 23)
+    want = cells.copy()
+    for i in range(len(cells)):
+        assert oracle.burn(want[i:i + 1], dt) == wr.SUCCESS
+    for i, name in enumerate(("internal_steps", "rhs_calls", "jacobian_calls", "decompositions", "linear_solves",
+                              "accepted_steps", "rejected_steps")):
+        assert (got[:, 15 + i] == want["stats"][name]).all(), name
+    assert got[:, :14].tobytes() == want["xn"].tobytes()
+    assert got[:, 14].tobytes() == want["e"].tobytes() and (got[:, 22] == wr.SUCCESS).all()
+    return want
+
+
+def test_advance(advance, tmp_path, oracle_port, wr):
+    """Cells with accepted and rejected attempts: alone in the warp, in pairs, one left over."""
+    cells = wr.make_batch_grid(3, 3)
+    want = burn(advance, tmp_path, oracle_port, wr, cells, 1e13)
+    assert want["stats"]["internal_steps"].sum() > want["stats"]["accepted_steps"].sum()

@@ -574,6 +574,7 @@ struct Kept {
             if (gl + t * G < NEQ * NEQ) m[t] = V[kE + gl + t * G];
 #pragma unroll
         for (int t = 0; t < K; ++t) f[t] = rhs[t];
+        __syncwarp();  // the caller changes the diagonal, whose entries other lanes have read here
     }
     __device__ __forceinline__ void restore(uint64_t* V, double (&rhs)[K], int gl) const {
 #pragma unroll 4
