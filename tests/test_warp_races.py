@@ -80,3 +80,31 @@ def test_advance(advance, tmp_path, oracle_port, wr):
     cells = wr.make_batch_grid(3, 3)
     want = burn(advance, tmp_path, oracle_port, wr, cells, 1e13)
     assert want["stats"]["internal_steps"].sum() > want["stats"]["accepted_steps"].sum()
+
+
+@pytest.fixture(scope="module")
+def gradient(built, tmp_path_factory):
+    unit = open(os.path.join(CSRC, "wr_diff_coop.cu")).read()
+    device = unit[:unit.index("template <class KernelT>")] + "}  // namespace\n}  // namespace diff\n}  // namespace wr\n"
+    return compile_program(tmp_path_factory.mktemp("gradient"), "gradient", device)
+
+
+def run_map(gradient, mode, tmp, oracle, cells, dts, log_mult):
+    mult = np.array([oracle.exp(p) for p in log_mult])
+    (tmp / "in").write_bytes(np.array([len(cells), len(dts)], np.int32).tobytes() + dts.tobytes() + mult.tobytes() +
+                             cells.tobytes())
+    run_program(gradient, mode, tmp / "in", tmp / "out")
+    out = np.frombuffer((tmp / "out").read_bytes()).reshape(len(cells), -1)
+    return out[:, :15], out[:, 15:30], out[:, 30:] * mult
+
+
+def test_forward_map(gradient, tmp_path, oracle_port, wr):
+    """Two cells one after the other in the warp, with rejected attempts: the oracle's final
+    states, bit for bit."""
+    from oracle import oracle as O
+    cells, dts = wr.make_batch_grid(3, 3)[1:], np.array([1e13, 2e13])
+    log_mult = np.random.default_rng(1).normal(0, 0.01, O.load_diff().num_multipliers)
+    rc, want, _, counts = O.load_diff().record(cells, dts, perturb=False, log_mult=log_mult)
+    assert rc == wr.SUCCESS
+    q, _, _ = run_map(gradient, "forward", tmp_path, oracle_port, cells, dts, log_mult)
+    assert q.tobytes() == want.tobytes()

@@ -112,6 +112,7 @@ __device__ __noinline__ int burn_record(uint64_t* V, double& yl, double tout, do
     coop::Kept<G, 1> kept;
 #pragma unroll 1
     for (;;) {
+        __syncwarp();  // every lane is done with the last attempt's factors and outputs in V
         const bool again = !fresh;  // the same state as the last attempt's
         if (fresh) {
             if (n_step > kMaxSteps) return WR_TOO_MANY_STEPS;
