@@ -86,13 +86,15 @@ def test_advance(advance, tmp_path, oracle_port, wr):
 def gradient(built, tmp_path_factory):
     unit = open(os.path.join(CSRC, "wr_diff_coop.cu")).read()
     device = unit[:unit.index("template <class KernelT>")] + "}  // namespace\n}  // namespace diff\n}  // namespace wr\n"
+    assert device.count("int first(int w) { ") == 1
+    device = device.replace("int first(int w) { ", "int first(int w) { program = w; ")
     return compile_program(tmp_path_factory.mktemp("gradient"), "gradient", device)
 
 
-def run_map(gradient, mode, tmp, oracle, cells, dts, log_mult):
+def run_map(gradient, mode, tmp, oracle, cells, dts, log_mult, qbar):
     mult = np.array([oracle.exp(p) for p in log_mult])
     (tmp / "in").write_bytes(np.array([len(cells), len(dts)], np.int32).tobytes() + dts.tobytes() + mult.tobytes() +
-                             cells.tobytes())
+                             cells.tobytes() + qbar.tobytes())
     run_program(gradient, mode, tmp / "in", tmp / "out")
     out = np.frombuffer((tmp / "out").read_bytes()).reshape(len(cells), -1)
     return out[:, :15], out[:, 15:30], out[:, 30:] * mult
@@ -106,5 +108,29 @@ def test_forward_map(gradient, tmp_path, oracle_port, wr):
     log_mult = np.random.default_rng(1).normal(0, 0.01, O.load_diff().num_multipliers)
     rc, want, _, counts = O.load_diff().record(cells, dts, perturb=False, log_mult=log_mult)
     assert rc == wr.SUCCESS
-    q, _, _ = run_map(gradient, "forward", tmp_path, oracle_port, cells, dts, log_mult)
+    q, _, _ = run_map(gradient, "forward", tmp_path, oracle_port, cells, dts, log_mult, np.zeros((2, 15)))
     assert q.tobytes() == want.tobytes()
+
+
+def test_adjoint(gradient, tmp_path, oracle_port, wr):
+    """The adjoint of the same map.  Its programs' slot array is larger than the forward
+    programs', and none of them may store into the slot that is the smaller array's sink
+    but to keep a value there.  Inner products with the tangent, <qbar, dq> = <ubar, du> +
+    <pbar, dp>, to 1e-8 of their terms as on the GPU, for the electrons, H, H2 and T (the
+    deuterium species, which start at 1e-40, end as rounding noise of the others)."""
+    from oracle import oracle as O
+    D, rng = O.load_diff(), np.random.default_rng(2)
+    cells, dts = wr.make_batch_grid(3, 3)[1:], np.array([1e13, 2e13])
+    log_mult = np.random.default_rng(1).normal(0, 0.01, D.num_multipliers)
+    rc, q, hbuf, counts = D.record(cells, dts, perturb=False, log_mult=log_mult)
+    assert rc == wr.SUCCESS
+    qbar = np.zeros((len(cells), 15))
+    for k in (0, 2, 8, 14):
+        qbar[:, k] = rng.normal(size=len(cells)) / q[:, k]
+    _, ubar, pbar = run_map(gradient, "adjoint", tmp_path, oracle_port, cells, dts, log_mult, qbar)
+    du = rng.normal(size=(len(cells), 15)) * np.concatenate([cells["xn"], cells["T"][:, None]], axis=1)
+    dp = rng.normal(size=D.num_multipliers)
+    rc, _, dq = D.tangent(cells, dts, hbuf, counts, du=du, dlog_mult=dp, perturb=False, log_mult=log_mult)
+    assert rc == wr.SUCCESS
+    terms = np.concatenate([ubar * du, pbar * dp], axis=1)
+    assert (np.abs((qbar * dq).sum(axis=1) - terms.sum(axis=1)) <= 1e-8 * np.abs(terms).sum(axis=1)).all()

@@ -1,8 +1,11 @@
 // The differentiation form's kernels (csrc/wr_diff_coop.cu: k_diff_forward and, with
 // "adjoint", k_diff_backward) on the CPU, one warp.  gradient forward|adjoint <in> <out>:
-// n, the number of outer steps, the timesteps, the multipliers and the cells' records ->
-// per cell q (15), the adjoint of u (15) and of the multipliers, for qbar = 1 / max(|q|, 1e-30).
+// n, the number of outer steps, the timesteps, the multipliers, the cells' records and qbar
+// (n x 15) -> per cell q (15), the adjoint of u (15) and of the multipliers.
 #include "warp_threads.h"
+
+// the lane's running program, which the test has Tab::first report
+inline thread_local int program;
 
 #include "device_code.h"
 
@@ -27,12 +30,14 @@ int main(int argc, char** argv) {
     ok = ok && std::fread(dt.data(), sizeof(double), steps, f) == dt.size();
     ok = ok && std::fread(mult.data(), sizeof(double), NP, f) == mult.size();
     ok = ok && std::fread(cells.data(), sizeof(wr_collapse_state), n, f) == cells.size();
+    std::vector<double> qbar(15 * n);
+    ok = ok && std::fread(qbar.data(), sizeof(double), 15 * n, f) == qbar.size();
     std::fclose(f);
     if (!ok) return 3;
     Args a{};
     a.cells = cells.data(), a.mult = mult.data(), a.dt_hist = dt.data();
     a.nsteps = steps, a.n = n, a.cap = cap, a.nseg = cap / kSeg + 1;
-    std::vector<double> ckpt(steps * kFields * n), hbuf(n * cap), q(15 * n), qbar(15 * n), ubar(15 * n),
+    std::vector<double> ckpt(steps * kFields * n), hbuf(n * cap), q(15 * n), ubar(15 * n),
         segck(n * a.nseg * wr::NEQ), ys(n * kSeg * wr::NEQ), stage(n * kSeg * kStage), mbar(n * NP);
     std::vector<int> counts(steps * n), status(n);
     std::vector<unsigned char> kind(steps * n);
@@ -46,10 +51,11 @@ int main(int argc, char** argv) {
     for (int s : status)
         if (s != WR_SUCCESS) return 4;
     if (adjoint) {
-        for (int i = 0; i < 15 * n; ++i) qbar[i] = 1.0 / std::max(std::fabs(q[i]), 1e-30);
         queue = 0;
-        // (the Jacobian and RHS programs, which the adjoint replays, have the smaller array's sink)
-        warp::is_sink = [](uint32_t addr) { return addr / 8 == cd::kNVA - 1; };
+        // the burn's replay runs the forward programs, whose sink is the smaller array's
+        warp::is_sink = [](uint32_t addr) {
+            return addr / 8 == (program < 2 * Tab::kRegimes ? Tab::kNV : cd::kNVA) - 1;
+        };
         warp::launch([&] { k_diff_backward(a); });
     }
     f = std::fopen(argv[3], "wb");

@@ -28,6 +28,7 @@ struct Tab {
     static __device__ __forceinline__ uint32_t ctl(int i) { return cp::kCtl[i]; }
     static __device__ __forceinline__ int first(int w) { return cp::kProgStep[w][0]; }
     static __device__ __forceinline__ int steps(int w) { return cp::kProgStep[w][1]; }
+    static __device__ __forceinline__ int sink(int) { return kNV - 1; }
     static __device__ __forceinline__ uint64_t regime(int k, int i) { return cp::kRegimeT[k][i]; }
     static __device__ __forceinline__ const uint16_t* out(int w) { return cp::kOut[w]; }
     static __device__ __forceinline__ const uint16_t* jac(int r) { return cp::kJac[r]; }

@@ -220,8 +220,8 @@ __device__ __noinline__ void run_prog(int which, int gl, uint64_t* V) {
     };
     uint32_t c0 = Tab::ctl(ctl0);
     operands(a.e[0], a.l[0]);
-    uint64_t res = 0;                         // the last step's main results,
-    uint32_t dst = vb + (Tab::kNV - 1) * 8;   // stored while this step's run
+    uint64_t res = 0;                          // the last step's main results,
+    uint32_t dst = vb + Tab::sink(which) * 8;  // stored while this step's run
     auto step = [&](const ulonglong2 e, uint32_t c, const ulonglong2 en, const uint64_t ln) {
         const uint32_t w1 = static_cast<uint32_t>(e.x >> 32);
         const uint32_t cls = c & CTL_CLASS;
@@ -592,9 +592,10 @@ struct KeepNothing {  // for a caller that never retries
 // Generated tables of one G, supplied by the translation unit that includes the
 // generated header (one unit per G keeps the large initialisers apart).
 //   Tab::kNV, Tab::kNR, Tab::kNF, Tab::kRegimes, Tab::kAdjoint and device accessors vconst(),
-//   vfun(), prog(), lit(), ctl(i) (control bytes of four steps), first(w) and steps(w)
-//   of program w = 2 * regime + kind, out(w) (RHS operands, then T), jac(regime) and
-//   regime(k, 0 or 1) (the temperatures between which regime k holds).
+//   vfun(), prog(), lit(), ctl(i) (control bytes of four steps), first(w), steps(w) and
+//   sink(w) (the slot that nothing reads) of program w = 2 * regime + kind, out(w) (RHS
+//   operands, then T), jac(regime) and regime(k, 0 or 1) (the temperatures between which
+//   regime k holds).
 
 }  // namespace coop
 

@@ -42,6 +42,9 @@ struct Tab {
     static __device__ __forceinline__ uint32_t ctl(int i) { return cd::kCtl[i]; }
     static __device__ __forceinline__ int first(int w) { return cd::kProgStep[w][0]; }
     static __device__ __forceinline__ int steps(int w) { return cd::kProgStep[w][1]; }
+    // the vector-Jacobian programs lie on the adjoint's larger slot array: kNV - 1 is one of
+    // their ordinary slots
+    static __device__ __forceinline__ int sink(int w) { return (w < 2 * kRegimes ? cd::kNV : cd::kNVA) - 1; }
     static __device__ __forceinline__ uint64_t regime(int k, int i) { return cd::kRegimeT[k][i]; }
     static __device__ __forceinline__ const uint16_t* out(int w) { return cd::kOut[w]; }
     static __device__ __forceinline__ const uint16_t* jac(int r) { return cd::kJac[r]; }
