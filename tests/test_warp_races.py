@@ -46,6 +46,7 @@ def run_program(exe, *args):
     races = sorted(set(re.findall(r"SUMMARY: ThreadSanitizer: data race (.*)", r.stderr)))
     assert not races, "\n".join(races[:20])
     assert r.returncode == 0, r.stderr[-2000:]
+    return r.stdout
 
 
 @pytest.fixture(scope="module", params=[8, 16, 32])
@@ -53,7 +54,8 @@ def advance(request, built, tmp_path_factory):
     G = request.param
     unit = open(os.path.join(CSRC, "wr_adv_coop.cuh")).read()
     tables = unit[unit.index("namespace cp ="):unit.index("static_assert(coop::kRes")].replace(
-        "WR_CAT(coop, WR_COOP_G)", f"coop{G}")
+        "WR_CAT(coop, WR_COOP_G)", f"coop{G}").replace("int first(int w) { ", "int first(int w) { started(w); ")
+    assert "started" in tables
     parts = f'#include "generated/coop_prog_g{G}.h"\n#include "wr_coop.cuh"\nnamespace wr {{\n{tables}\n}}\n'
     return compile_program(tmp_path_factory.mktemp(f"advance{G}"), "advance", parts)
 
@@ -62,24 +64,42 @@ def burn(advance, tmp, oracle, wr, cells, dt):
     rec = np.zeros((len(cells), 16))
     rec[:, :14], rec[:, 14], rec[:, 15] = cells["xn"], cells["T"], dt
     (tmp / "in").write_bytes(rec.tobytes())
-    run_program(advance, tmp / "in", tmp / "out")
+    programs = [int(w) for w in run_program(advance, tmp / "in", tmp / "out").split()]
     got = np.frombuffer((tmp / "out").read_bytes()).reshape(-1, 23)
     want = cells.copy()
     for i in range(len(cells)):
-        assert oracle.burn(want[i:i + 1], dt) == wr.SUCCESS
+        assert oracle.burn(want[i:i + 1], np.broadcast_to(dt, len(cells))[i]) == wr.SUCCESS
     for i, name in enumerate(("internal_steps", "rhs_calls", "jacobian_calls", "decompositions", "linear_solves",
                               "accepted_steps", "rejected_steps")):
         assert (got[:, 15 + i] == want["stats"][name]).all(), name
     assert got[:, :14].tobytes() == want["xn"].tobytes()
     assert got[:, 14].tobytes() == want["e"].tobytes() and (got[:, 22] == wr.SUCCESS).all()
-    return want
+    return want["stats"], programs
 
 
 def test_advance(advance, tmp_path, oracle_port, wr):
     """Cells with accepted and rejected attempts: alone in the warp, in pairs, one left over."""
     cells = wr.make_batch_grid(3, 3)
-    want = burn(advance, tmp_path, oracle_port, wr, cells, 1e13)
-    assert want["stats"]["internal_steps"].sum() > want["stats"]["accepted_steps"].sum()
+    stats, _ = burn(advance, tmp_path, oracle_port, wr, cells, 1e13)
+    assert stats["internal_steps"].sum() > stats["accepted_steps"].sum()
+
+
+@pytest.mark.parametrize("order", [(0, 1), (1, 0)])
+def test_group_without_cell_follows(advance, tmp_path, oracle_port, wr, order):
+    """A cell that retries beside a group whose own cell is done: the group without a cell
+    computes the other's attempts, so the warp's programs are those of the cell alone but
+    for one Jacobian at the new company (at one cell per warp, of the cell alone)."""
+    cells = wr.make_batch_grid(3, 2)
+    cells[1]["xn"] *= 1e12  # dense and hot: stages from its rates are far from the cold cell's state
+    both = [cells[list(order)], np.array([1e14, 1e-5])[list(order)]]  # five attempts (two rejected) and one
+    stats, programs = burn(advance, tmp_path, oracle_port, wr, *both)
+    assert (stats["internal_steps"] == np.array([5, 1])[list(order)]).all()
+    _, alone = burn(advance, tmp_path, oracle_port, wr, cells[:1], 1e14)
+    if len(programs) >= len(alone) + 3:  # one after the other
+        want = alone + programs[len(alone):] if order == (0, 1) else programs[:-len(alone)] + alone
+    else:
+        want = programs[:3] + alone[:1] + alone[3:]
+    assert programs == want
 
 
 @pytest.fixture(scope="module")

@@ -1,8 +1,14 @@
 // The cooperative advance (csrc/wr_coop.cuh: k_advance_coop) on the CPU, one warp of
 // 8, 16 or 32 lanes per cell.  advance <in> <out>: records of 16 doubles (14 number
 // densities, T, the timestep) -> records of 23: the burned number densities and energy, the
-// seven counters and the launch's failure code.
+// seven counters and the launch's failure code.  The programs that the warp ran, in order,
+// go to standard output.
 #include "warp_threads.h"
+
+// called by Tab::first, which the test has report the program it starts
+inline void started(int program) {
+    if (threadIdx.x == 0) std::printf("%d\n", program);
+}
 
 #include "device_code.h"
 

@@ -810,6 +810,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
     bool have = false;     // the group holds a cell
     bool drained = false;  // it has seen the queue's end
     int regime = 0;        // the temperature regime of its last evaluation
+    int kept_of = slot;    // the group whose state `kept` is of
     double y[K];
     Kept<G, K> kept;
 #pragma unroll
@@ -898,8 +899,9 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
         // follows one that has one (same state, same branches) and commits nothing
         const unsigned holders = __ballot_sync(kWarp, have);
         if (holders == 0) break;
+        const int leader = (__ffs(holders) - 1) / G;
         {
-            const int from = (__ffs(holders) - 1) / G * G + gl;
+            const int from = leader * G + gl;
 #pragma unroll
             for (int t = 0; t < K; ++t) {
                 const double o = __shfl_sync(kWarp, y[t], from);
@@ -914,8 +916,13 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
         pc.attempt();
 
         // a rejected attempt is retried from the same state: where no cell of the warp is
-        // at a new one, the Jacobian and the RHS of the last attempt stand
-        const bool again = !__any_sync(kWarp, have && L.fresh);
+        // at a new one, the Jacobian and the RHS of the last attempt stand.  A group that has
+        // begun to follow another has its own last cell's: from them its stages would go
+        // elsewhere, out of the temperature regime, and the warp's vote would run the general
+        // program for everyone at every retry.
+        const int state_of = have ? slot : leader;
+        const bool again = !__any_sync(kWarp, (have && L.fresh) || state_of != kept_of);
+        kept_of = state_of;
         if (L.fresh) L.n_jac += 1;
         L.fresh = false;
         const double h = L.h;
