@@ -33,12 +33,13 @@ def test_cta32_shapes(wr, gpu, sms, oracle_port, tiles, math):
     def steps(part, dts=None):
         out, taken, t = part.copy(), [], 0.0
         with wr.Context(len(out), 0, math) as ctx:
-            ctx.set_policy(wr.POLICY_GRIDWIDE_CTA32)
             ctx.upload(out)
             for k in range(3):
+                ctx.set_policy(wr.POLICY_GRIDWIDE_INDEPENDENT)  # the two policies' prepare is the same
                 rc, dt = ctx.prepare(k, t, k, True)
                 assert rc == wr.SUCCESS
                 dt = dt if dts is None else dts[k]
+                ctx.set_policy(wr.POLICY_GRIDWIDE_CTA32)
                 rc, moved = ctx.advance(k, t + dt, dt)
                 assert rc == wr.SUCCESS and moved == len(out)
                 taken.append(dt)
