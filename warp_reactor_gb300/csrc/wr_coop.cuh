@@ -806,11 +806,10 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
 
     PhaseClock<PH> pc;
     Lane L;
-    int cell = -1, g = 0;
+    int cell = INT_MIN, g = 0;  // without a cell: -1 - (the group it follows)
     bool have = false;     // the group holds a cell
     bool drained = false;  // it has seen the queue's end
     int regime = 0;        // the temperature regime of its last evaluation
-    int kept_of = slot;    // the group whose state `kept` is of
     double y[K];
     Kept<G, K> kept;
 #pragma unroll
@@ -920,9 +919,9 @@ __global__ void __launch_bounds__(W * 32, 1) k_advance_coop(DevState s, StepCtl*
         // begun to follow another has its own last cell's: from them its stages would go
         // elsewhere, out of the temperature regime, and the warp's vote would run the general
         // program for everyone at every retry.
-        const int state_of = have ? slot : leader;
-        const bool again = !__any_sync(kWarp, (have && L.fresh) || state_of != kept_of);
-        kept_of = state_of;
+        const bool joins = !have && cell != -1 - leader;
+        const bool again = !__any_sync(kWarp, have ? L.fresh : joins);
+        if (joins) cell = -1 - leader;
         if (L.fresh) L.n_jac += 1;
         L.fresh = false;
         const double h = L.h;
