@@ -28,7 +28,10 @@ namespace {
 thread_local std::string g_last_error;
 std::atomic<uint64_t> g_launches{0};
 
+// reports an error and clears it: the runtime keeps a failed allocation's as its last
+// error, where the check after the next launch, of any context, would find it
 int fail(const char* what, cudaError_t e) {
+    cudaGetLastError();
     g_last_error = std::string(what) + ": " + cudaGetErrorString(e);
     return WR_BAD_INPUTS;
 }

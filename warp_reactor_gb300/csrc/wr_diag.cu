@@ -120,6 +120,7 @@ struct DevBuf {
 };
 
 int diag_fail(const char* what, cudaError_t e) {
+    cudaGetLastError();  // reported here: not the next launch check's
     g_diag_error = std::string(what) + ": " + cudaGetErrorString(e);
     return WR_BAD_INPUTS;
 }

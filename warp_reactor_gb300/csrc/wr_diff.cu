@@ -60,6 +60,7 @@ int fail(wr_diff* d, const std::string& msg, int code = WR_BAD_INPUTS) {
 
 bool cuda_ok(wr_diff* d, cudaError_t e, const char* what) {
     if (e == cudaSuccess) return true;
+    cudaGetLastError();  // reported here: not the next launch check's
     if (d) d->error = std::string(what) + ": " + cudaGetErrorString(e);
     return false;
 }

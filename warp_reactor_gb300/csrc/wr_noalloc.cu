@@ -62,6 +62,10 @@ int noalloc_fail(const std::string& msg) {
     g_noalloc_error = msg;
     return WR_BAD_INPUTS;
 }
+int noalloc_fail(const char* what, cudaError_t e) {
+    cudaGetLastError();  // reported here: not the next launch check's
+    return noalloc_fail(std::string(what) + ": " + cudaGetErrorString(e));
+}
 
 __global__ void k_noalloc_unpack(const wr_collapse_state* __restrict__ in, DevState s, StepCtl* ctl, int cgs,
                                  double next_grid_time, double dt_grid) {
@@ -129,18 +133,18 @@ __global__ void k_noalloc_pack(DevState s, wr_collapse_state* __restrict__ out) 
 int scratch_address(void** out) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return noalloc_fail(std::string("cudaGetDevice: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) return noalloc_fail("cudaGetDevice", e);
     if (dev < 0 || dev >= kMaxDevices) return noalloc_fail("wr_advance_cells_noalloc: device index out of range");
     std::lock_guard<std::mutex> lock(g_mu);
     if (!g_scratch_ptr[dev]) {
         void* p = nullptr;
         e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess || !p)
-            return noalloc_fail(std::string("cudaGetSymbolAddress(scratch): ") + cudaGetErrorString(e));
+            return noalloc_fail("cudaGetSymbolAddress(scratch)", e);
         e = configure_advance_coop16();  // dynamic shared memory limits of the advance kernels
         if (e == cudaSuccess) e = configure_advance_coop32();
         if (e != cudaSuccess)
-            return noalloc_fail(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+            return noalloc_fail("cudaFuncSetAttribute", e);
         g_scratch_ptr[dev] = p;
     }
     *out = g_scratch_ptr[dev];
@@ -198,7 +202,7 @@ int wr_advance_cells_noalloc(wr_collapse_state* d_cells, int num_cells, int comp
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess)
-        return noalloc_fail(std::string("wr_advance_cells_noalloc: device query: ") + cudaGetErrorString(e));
+        return noalloc_fail("wr_advance_cells_noalloc: device query", e);
 
     const int grid = (num_cells + 255) / 256;
     k_noalloc_unpack<<<grid, 256>>>(d_cells, s, ctl, completed_global_steps, next_grid_time, dt_grid);
@@ -216,7 +220,7 @@ int wr_advance_cells_noalloc(wr_collapse_state* d_cells, int num_cells, int comp
     if (e == cudaSuccess)
         e = cudaMemcpy(head, &ctl->failure, sizeof(head), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess)
-        return noalloc_fail(std::string("wr_advance_cells_noalloc: ") + cudaGetErrorString(e));
+        return noalloc_fail("wr_advance_cells_noalloc", e);
     *integrated_out = head[1];
     return head[0];
 }
