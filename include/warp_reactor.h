@@ -194,8 +194,12 @@ int wr_set_profiling(wr_ctx* ctx, int on);
  * triangular solves with a group of lanes (generated vector programs, a
  * warp-cooperative LU with shuffle pivot search, shared-memory matrices).
  * Variants 0-2 and 4-7 give identical results (only the speed differs); variant
- * 3 approximates the FP64 result.  No reference counterpart (the reference fixes
- * one thread per cell, 128 threads per block, reproducer.cpp:7398). */
+ * 3 approximates the FP64 result.  Variants 0-4 have scratch of their own (210 MB on 152
+ * SMs), allocated by the first wr_run, wr_advance or wr_autotune that launches one of
+ * them: that call may fail for want of memory, which leaves the context usable with the
+ * other variants, and may not fall inside a stream capture of its thread; this one asks
+ * the device for nothing.  No reference counterpart (the reference fixes one thread per
+ * cell, 128 threads per block, reproducer.cpp:7398). */
 int wr_set_advance_variant(wr_ctx* ctx, int variant);
 
 /* Autotuner: times the first `steps` outer steps of the uploaded state with each

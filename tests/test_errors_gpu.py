@@ -1,4 +1,8 @@
-"""Calls after a failed one: an error is reported by the call that met it and by no other."""
+"""Calls after a failed or an awkward one: an error is reported by the call that met it and
+by no other, and choosing a launch shape asks the device for nothing."""
+import ctypes
+import os
+
 import numpy as np
 import pytest
 
@@ -32,3 +36,22 @@ def test_failed_allocation_leaves_other_calls_alone(wr, gpu):
         wr.Context(2**31 - 1)
     with wr.Context(len(cells)) as ctx:
         assert step(ctx, cells) == want
+
+def test_choosing_a_shape_during_a_capture(wr, gpu):
+    """A program may choose a context's launch shape while it captures a stream of its own."""
+    try:
+        cudart = ctypes.CDLL("libcudart.so")
+    except OSError:
+        from warp_reactor_gb300 import build
+        cudart = ctypes.CDLL(os.path.join(build._cuda_home(), "lib64", "libcudart.so"))
+    cells = wr.make_grid(2)
+    with wr.Context(len(cells)) as ctx:
+        want = step(ctx, cells)
+    stream, graph = ctypes.c_void_p(), ctypes.c_void_p()
+    with wr.Context(len(cells)) as ctx:
+        assert cudart.cudaStreamCreateWithFlags(ctypes.byref(stream), 1) == 0  # non-blocking
+        assert cudart.cudaStreamBeginCapture(stream, 1) == 0                   # this thread's calls
+        ctx.set_variant(2)
+        assert cudart.cudaStreamEndCapture(stream, ctypes.byref(graph)) == 0
+        assert step(ctx, cells) == want
+    assert cudart.cudaGraphDestroy(graph) == 0 and cudart.cudaStreamDestroy(stream) == 0

@@ -561,11 +561,12 @@ static int ensure_staging(wr_ctx* ctx) {
     return e == cudaSuccess ? WR_SUCCESS : fail("cudaMalloc(staging)", e);
 }
 
-// the lane-per-cell shapes' Jacobian backup and iteration matrices, allocated when one
-// of these shapes is first chosen (two times 105 MB that the cooperative advance never
-// touches: half the time of a context's creation)
+// the lane-per-cell shapes' Jacobian backup and iteration matrices, allocated by the first
+// call that launches one of them (two times 105 MB that the cooperative advance never
+// touches: half the time of a context's creation).  Not where the shape is chosen: choosing
+// it asks the device for nothing, so it may fall inside a stream capture and cannot fail.
 static int ensure_lane_scratch(wr_ctx* ctx) {
-    if (ctx->ebuf) return WR_SUCCESS;
+    if (ctx->ebuf || ctx->policy == WR_POLICY_GRIDWIDE_CTA32 || is_coop(ctx->variant)) return WR_SUCCESS;
     size_t nslots = 0;  // lane slots of the largest configuration
     for (const AdvanceShape& sh : kAdvanceShapes) {
         const size_t slots = static_cast<size_t>(ctx->sms) * sh.blocks_per_sm * sh.threads;
@@ -630,6 +631,7 @@ int wr_advance(wr_ctx* ctx, int completed_global_steps, double next_grid_time, d
     if (!ctx || !integrated_out) return fail_msg("wr_advance: null argument");
     if (ctx->G != 1) return fail_msg("wr_advance: host-stepped calls need a one-grid context");
     int rc = set_device(ctx);
+    if (rc == WR_SUCCESS) rc = ensure_lane_scratch(ctx);
     if (rc != WR_SUCCESS) return rc;
     g_launches.fetch_add(1, std::memory_order_relaxed);
     k_begin_advance<<<1, 1, 0, ctx->stream>>>(ctx->ctl, completed_global_steps, next_grid_time, dt_grid);
@@ -701,7 +703,8 @@ static int ensure_graph(wr_ctx* ctx) {
 // records an event pair around every prepare and advance launch, and an event
 // pair brackets the whole run: the per-kernel times of the shipped path.
 static int run_graph(wr_ctx* ctx, int perturb, int* completed_global_steps) {
-    int rc = ensure_graph(ctx);
+    int rc = ensure_lane_scratch(ctx);
+    if (rc == WR_SUCCESS) rc = ensure_graph(ctx);
     if (rc != WR_SUCCESS) return rc;
     const int nev = 4 * WR_MAX_COLLAPSE_STEPS + 2;
     wr_run_timing t{};
@@ -757,7 +760,8 @@ int wr_run(wr_ctx* ctx, int perturb, int* completed_global_steps) {
 // launch by launch, with CUDA events around every kernel when profiling; stops
 // after max_steps outer steps (the autotuner's short runs)
 static int run_profiled(wr_ctx* ctx, int perturb, int max_steps, int* completed_global_steps) {
-    int rc = WR_SUCCESS;
+    int rc = ensure_lane_scratch(ctx);
+    if (rc != WR_SUCCESS) return rc;
     g_launches.fetch_add(1, std::memory_order_relaxed);
     const int nev = 4 * WR_MAX_COLLAPSE_STEPS + 2;
     ctx->ev_used = 0;
@@ -841,7 +845,6 @@ int wr_grid_dt_history(wr_ctx* ctx, int grid, double* out, int max_steps) {
 int wr_autotune(wr_ctx* ctx, int perturb, int steps, int* best_variant) {
     if (!ctx || !best_variant || steps < 1) return fail_msg("wr_autotune: bad argument");
     int rc = set_device(ctx);
-    if (rc == WR_SUCCESS) rc = ensure_lane_scratch(ctx);  // it times the lane-per-cell shapes too
     if (rc != WR_SUCCESS) return rc;
     const size_t bytes = static_cast<size_t>(ctx->n) * ((3 + NS + 2) * sizeof(double) + 7 * sizeof(uint64_t) + 4 * sizeof(int));
     void* snap = nullptr;
@@ -906,11 +909,6 @@ int wr_set_policy(wr_ctx* ctx, int policy) {
 int wr_set_advance_variant(wr_ctx* ctx, int variant) {
     if (!ctx) return fail_msg("wr_set_advance_variant: null context");
     if (variant < 0 || variant >= kAdvanceVariants) return fail_msg("wr_set_advance_variant: unknown variant");
-    if (!is_coop(variant)) {
-        int rc = set_device(ctx);
-        if (rc == WR_SUCCESS) rc = ensure_lane_scratch(ctx);
-        if (rc != WR_SUCCESS) return rc;
-    }
     ctx->variant = variant;
     return WR_SUCCESS;
 }
