@@ -184,23 +184,28 @@ def algorithmic_ops(cells):
 
 
 def program_figures(G=16):
-    """Figures of the default advance's generated vector programs (16 lanes per
-    cell, two cells per warp) per ROS2S attempt of one warp: steps and FP64 issue
-    slots of one Jacobian+RHS and two RHS programs, the slots per cell, and the
-    shared-memory wavefronts their slot accesses take per half warp against one
-    per access (coop.shared_wavefronts: the bank-conflict model)."""
+    """Figures of the 16-lane advance's generated vector programs (two cells per warp) per
+    ROS2S attempt of one warp: the steps it executes and the FP64 issue slots of one
+    Jacobian+RHS and two RHS programs, and the shared-memory wavefronts their slot
+    accesses take per half warp against one per access (coop.shared_wavefronts: the
+    bank-conflict model).  "general": the programs for any state; "regimes": those of one
+    temperature range (K), which a warp runs when its cells' temperatures share one."""
     from warp_reactor_gb300.gen import coop, ir_io
-    g = coop.generate(G, ir_io.load())
-    out = {"lanes_per_cell": G, "slots_per_cell": g["nv"], "warps_per_sm": g["warps"], "steps": 0,
-           "fp64_issue_slots": 0.0, "shared_wavefronts": 0, "shared_accesses": 0}
-    for kind, runs in (("jrhs", 1), ("rhs", 2)):
-        pr = g["progs"][kind]
-        w = coop.shared_wavefronts(pr)
-        out["steps"] += runs * pr["nsteps"]  # as executed: padded to a multiple of four
-        out["fp64_issue_slots"] += runs * pr["stats"]["fp64_slots"]
-        out["shared_wavefronts"] += runs * w["wavefronts"]
-        out["shared_accesses"] += runs * w["ideal"]
-    return out
+    g = coop.generate(G, ir_io.load(), regimes=coop.REGIMES)
+
+    def per_attempt(progs):
+        out = {"steps": 0, "fp64_issue_slots": 0.0, "shared_wavefronts": 0, "shared_accesses": 0}
+        for kind, runs in (("jrhs", 1), ("rhs", 2)):
+            w = coop.shared_wavefronts(progs[kind])
+            out["steps"] += runs * (len(coop.device_words(progs[kind], g["nv"])[0]) - coop.PREFETCH_PAD)
+            out["fp64_issue_slots"] += runs * progs[kind]["stats"]["fp64_slots"]
+            out["shared_wavefronts"] += runs * w["wavefronts"]
+            out["shared_accesses"] += runs * w["ideal"]
+        return out
+
+    return {"lanes_per_cell": G, "slots_per_cell": g["nv"], "warps_per_sm": g["warps"],
+            "general": per_attempt(g["progs"]),
+            "regimes": [{"T_above": r["lo"], "T_to": r["hi"], **per_attempt(r["progs"])} for r in g["regimes"]]}
 
 
 def precision_form(wr, device, math_mode, grid=16, steps=300):

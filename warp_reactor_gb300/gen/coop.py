@@ -1266,15 +1266,15 @@ def generate(G: int, dag=None, limit="default", tune="default", banked="default"
 
 
 def shared_wavefronts(pr: dict) -> dict:
-    """Shared-memory wavefronts of one encoded program's slot accesses, per half
-    warp, by operand (X, Y, Z, D of the main word; A, B, C, D2 of the integer word),
-    against one wavefront per access.  A 64-bit access of a half warp (one cell's
+    """Shared-memory wavefronts of one program's slot accesses, per half warp, by
+    operand (X, Y, Z, D of the main word; A, B, C, D2 of the integer word), against one
+    wavefront per access.  A 64-bit access of a half warp (one cell's
     G = 16 lanes) is conflict-free when its distinct slots lie in distinct bank
     pairs (slot mod 16: the cell's array base is uniform over the half warp);
     otherwise it takes as many wavefronts as the most-used bank pair holds distinct
-    slots.  Accesses follow the interpreter: an FMA step loads X, Y, Z; exp, log
-    and sqrt load Y, division X and Y; every non-idle step stores D; a step with
-    integer nodes loads A, B, C and stores D2."""
+    slots.  Accesses follow the interpreter on the device's words: every step loads X,
+    Y and Z and stores D, twice where it flushes; a step with integer nodes loads A, B
+    and C and stores D2."""
     def wf(slots):
         by = collections.defaultdict(set)
         for s in slots:
@@ -1285,12 +1285,10 @@ def shared_wavefronts(pr: dict) -> dict:
         return ((w >> (16 * k)) & 0xffff) >> 3
 
     got, ideal = collections.Counter(), collections.Counter()
-    for lanes in pr["words"][:pr["nsteps"]]:
-        m0 = lanes[0][0]
-        cls, flint = (m0 >> 48) & 7, (m0 >> 32) & FL_INT
-        used = {C_FMA: "XYZD", C_DIV: "XYD"}.get(cls, "YD" if cls != C_NONE else "")
-        acc = [(n, [field(m, "XYZD".index(n)) for m, _, _ in lanes]) for n in used]
-        if flint:
+    words, ctl = device_words(pr, MAX_SLOTS)
+    for lanes, c in zip(words[:len(words) - PREFETCH_PAD], ctl):
+        acc = [(n, [field(m, "XYZD".index(n)) for m, _, _ in lanes]) for n in ("XYZDD" if c & CTL_FLUSH else "XYZD")]
+        if c & CTL_INT:
             acc += [(n, [field(i, k) for _, i, _ in lanes]) for k, n in enumerate(("A", "B", "C", "D2"))]
         for n, slots in acc:
             got[n] += wf(slots)
