@@ -11,6 +11,7 @@ import pytest
 
 HERE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "warp_threads")
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "warp_reactor_gb300", "csrc")
+INCLUDE = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "include")
 
 # the PTX accesses of wr_coop.cuh, in C++
 PTX = {
@@ -21,20 +22,29 @@ PTX = {
 }
 
 
-def compile_program(tmp, name, parts, flags=()):
+def compile_program(tmp, name, parts):
     """``name``.cpp with the device code ``parts`` as device_code.h, under the sanitizer."""
-    src = open(os.path.join(CSRC, "wr_coop.cuh")).read()
-    for asm, cxx in PTX.items():
-        assert src.count(asm) == 1, asm
-        src = src.replace(asm, cxx)
-    assert "asm" not in src
-    (tmp / "wr_coop.cuh").write_text(src)
+    for header in ("wr_coop.cuh", "wr_kernels.cuh", "wr_physics.cuh", "wr_math.h", "wr_diff.cuh"):
+        src = open(os.path.join(CSRC, header)).read().replace('"../../include/', f'"{INCLUDE}/')
+        if header == "wr_coop.cuh":
+            for asm, cxx in PTX.items():
+                assert src.count(asm) == 1, asm
+                src = src.replace(asm, cxx)
+            assert "asm" not in src
+        if header == "wr_math.h":
+            host = "#else\n    return a / b;\n#endif"
+            assert src.count(host) == 1
+            src = src.replace(host, host.replace("a / b", "native_division(a, b)"))
+        (tmp / header).write_text(src)
     (tmp / "cuda_runtime.h").write_text("#pragma once\nusing cudaError_t = int;\nusing cudaStream_t = void*;\n")
     (tmp / "device_code.h").write_text(parts)
     exe = str(tmp / name)
-    subprocess.run(["g++", "-std=c++17", "-O1", "-g", "-fsanitize=thread", "-ffp-contract=off", "-fno-inline-small-functions",
-                    "-Wno-unknown-pragmas", "-I", str(tmp), "-I", HERE, "-I", CSRC, *flags,
-                    os.path.join(HERE, name + ".cpp"), "-o", exe, "-pthread"], check=True)
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-g", "-fsanitize=thread", "-ffp-contract=off", "-Wno-unknown-pragmas",
+                        "-I", str(tmp), "-I", HERE, "-I", CSRC, os.path.join(HERE, name + ".cpp"), "-o", exe, "-pthread"],
+                       capture_output=True, text=True)
+    if "tsan" in r.stderr and "cannot find" in r.stderr:
+        pytest.skip("no ThreadSanitizer runtime here")
+    assert r.returncode == 0, r.stderr[-4000:]
     return exe
 
 
@@ -100,6 +110,26 @@ def test_group_without_cell_follows(advance, tmp_path, oracle_port, wr, order):
     else:
         want = programs[:3] + alone[:1] + alone[3:]
     assert programs == want
+
+
+@pytest.fixture(scope="module")
+def controller(tmp_path_factory):
+    return compile_program(tmp_path_factory.mktemp("controller"), "controller", "")
+
+
+@pytest.mark.parametrize("err,erracc,hacc,h", [(0.3, 1.0, 0.0, 1e11), (40.0, 1.0, 0.0, 1e13), (1e-7, 1.0, 0.0, 3e5),
+                                               (0.7, 1e-2, 2e10, 3e10), (2.5, 0.4, 1e9, 4e9)])
+def test_controller(controller, oracle_port, err, erracc, hacc, h):
+    """Both step sizes of the reference's controller (reproducer.cpp:7308-7327), in every
+    lane; the first attempts of a burn (no accepted step yet) divide on the integer path."""
+    out = run_program(controller, err, erracc, hacc, h).split()
+    sizes = np.array([float.fromhex(v) for v in out[:-1]]).reshape(-1, 2)
+    fac = max(1 / 6.0, min(1 / 0.2, oracle_port.cbrt(err) / 0.9))
+    assert (sizes[:, 0] == h / fac).all()
+    if hacc != 0.0:
+        gus = max(1 / 6.0, min(1 / 0.2, hacc / h * oracle_port.cbrt(err * err / erracc) / 0.9))
+        assert (sizes[:, 1] == h / max(fac, gus)).all()
+    assert int(out[-1]) == 0
 
 
 @pytest.fixture(scope="module")

@@ -201,6 +201,13 @@ inline unsigned long long atomicMin(unsigned long long* p, unsigned long long v)
     if (v < old) *p = v;
     return old;
 }
+// the fallback of wr_div_finish, counted
+inline thread_local int native_divisions = 0;
+inline double native_division(double a, double b) {
+    ++native_divisions;
+    return a / b;
+}
+
 // shared-window addresses: byte offsets from the program's slot array
 inline uint64_t* slots = nullptr;
 inline size_t __cvta_generic_to_shared(const uint64_t* p) { return static_cast<size_t>(p - slots) * 8; }

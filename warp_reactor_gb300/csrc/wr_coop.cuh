@@ -772,7 +772,10 @@ __device__ __forceinline__ void step_sizes(double err, double erracc, double hac
                                            double& hnew, double& hgus) {
     using coop::kWarp;
     const bool odd = (gl & 1) != 0;
-    const double q = ddiv(odd ? hacc : err * err, odd ? h : erracc);
+    // before the first accepted step (hacc 0) hgus is not used, and a zero would take the
+    // odd lanes through the division's native fallback beside the even lanes' quotient: 7 k
+    // cycles of every first attempt, a 64^3 collapse 23.56 s instead of 23.20 s
+    const double q = ddiv(odd ? (hacc == 0.0 ? h : hacc) : err * err, odd ? h : erracc);
     const double e2 = __shfl_sync(kWarp, q, 0, G), ratio = __shfl_sync(kWarp, q, 1, G);
     const double c = cbrt(odd ? e2 : err);
     const double raw = ddiv(odd ? ratio * c : c, kSafe);
