@@ -1,5 +1,6 @@
 """Calls after a failed or an awkward one: an error is reported by the call that met it and
-by no other, and choosing a launch shape asks the device for nothing."""
+by no other, choosing a launch shape asks the device for nothing, and the launch counter
+counts every entry point's kernels."""
 import ctypes
 import os
 
@@ -55,3 +56,28 @@ def test_choosing_a_shape_during_a_capture(wr, gpu):
         assert cudart.cudaStreamEndCapture(stream, ctypes.byref(graph)) == 0
         assert step(ctx, cells) == want
     assert cudart.cudaGraphDestroy(graph) == 0 and cudart.cudaStreamDestroy(stream) == 0
+
+
+def test_launch_count(wr, gpu):
+    """wr_kernel_launch_count over the entry points that launch kernels of their own."""
+    import torch
+    from warp_reactor_gb300 import diff
+    cells = wr.make_grid(2)
+    with wr.Context(len(cells), 0, wr.MATH_PORTABLE) as ctx:
+        ctx.upload(cells)
+        _, dt = ctx.prepare(0, 0.0, 0, True)
+    records = torch.from_numpy(cells.view(np.uint8).copy()).cuda()
+    q = torch.empty(len(cells), 15, dtype=torch.float64, device="cuda")
+    p = torch.empty(diff.num_multipliers(), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    f, moved = wr.lib().wr_advance_cells_noalloc, ctypes.c_int()
+    f.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_double, ctypes.c_double,
+                  ctypes.POINTER(ctypes.c_int)]
+    with diff.DiffMap(len(cells), max_outer_steps=1) as dmap:
+        before = wr.kernel_launch_count()
+        dmap.forward(records, None, None, [dt], False, q)
+        dmap.backward(torch.ones_like(q), torch.empty_like(q), p)
+        assert wr.kernel_launch_count() - before == 4  # multipliers, forward; backward, their sum
+    before = wr.kernel_launch_count()
+    assert f(records.data_ptr(), len(cells), 0, dt, dt, ctypes.byref(moved)) == wr.SUCCESS
+    assert wr.kernel_launch_count() - before == 5      # unpack, queue, advance, commit, pack

@@ -219,6 +219,8 @@ __global__ void __launch_bounds__(256) k_commit(DevState s, StepCtl* ctl) {
     }
 }
 
+void count_launches(int n) { g_launches.fetch_add(static_cast<uint64_t>(n), std::memory_order_relaxed); }
+
 cudaError_t launch_order_preburn(cudaStream_t stream, DevState s, StepCtl* ctl) {
     g_launches.fetch_add(1, std::memory_order_relaxed);
     k_order_preburn<<<(s.n + 255) / 256, 256, 0, stream>>>(s, ctl);

@@ -6,6 +6,7 @@
 #include <string>
 
 #include "wr_diff.cuh"
+#include "wr_launch.h"
 
 namespace wr {
 namespace diff {
@@ -168,6 +169,7 @@ int wr_diff_forward(wr_diff* d, const wr_collapse_state* d_cells, const double* 
     wr::diff::Args a = make_args(d);
     a.q = d_q;
     if (!cuda_ok(d, wr::diff::launch_diff_forward(a, d->sms, d->stream), "k_diff_forward launch")) return WR_BAD_INPUTS;
+    wr::count_launches(2);
     if (!cuda_ok(d, cudaStreamSynchronize(d->stream), "k_diff_forward")) return WR_BAD_INPUTS;
     // first failing cell in index order decides the result
     int* st = new int[d->n];
@@ -195,6 +197,7 @@ int wr_diff_backward(wr_diff* d, const double* d_qbar, double* d_ubar, double* d
     if (!cuda_ok(d, wr::diff::launch_diff_backward(a, d->sms, d->stream), "k_diff_backward launch"))
         return WR_BAD_INPUTS;
     wr::diff::k_diff_reduce<<<1, 64, 0, d->stream>>>(d->mbar, d->mult, d->n, d_pbar);
+    wr::count_launches(2);
     if (!cuda_ok(d, cudaStreamSynchronize(d->stream), "k_diff_backward")) return WR_BAD_INPUTS;
     return WR_SUCCESS;
 }

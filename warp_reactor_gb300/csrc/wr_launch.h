@@ -91,6 +91,8 @@ cudaError_t launch_advance_coop32(int math_cuda, int blocks, cudaStream_t stream
 // and the commit of the cells it burned
 cudaError_t launch_order_preburn(cudaStream_t stream, DevState s, StepCtl* ctl);
 cudaError_t launch_commit(cudaStream_t stream, DevState s, StepCtl* ctl);
+// kernels launched outside wr_capi.cu, for wr_kernel_launch_count
+void count_launches(int n);
 // diagnostics of the cooperative programs and LU on device buffers (wr_diag.cu)
 cudaError_t diag_coop_network8(int math_cuda, int n, const double* y, double* J, double* f, double* f2);
 cudaError_t diag_coop_network16(int math_cuda, int n, const double* y, double* J, double* f, double* f2);

@@ -215,6 +215,7 @@ int wr_advance_cells_noalloc(wr_collapse_state* d_cells, int num_cells, int comp
     if (e == cudaSuccess) {
         k_noalloc_pack<<<grid, 256>>>(s, d_cells);
         e = cudaGetLastError();
+        count_launches(3);  // unpack, the advance, pack: the other two count themselves
     }
     int head[2] = {0, 0};  // failure, integrated (adjacent ints of StepCtl)
     if (e == cudaSuccess)
