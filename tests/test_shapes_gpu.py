@@ -3,6 +3,7 @@ purpose (sizes follow the device's SM count) and compared with another implement
 the CPU oracle, the lane-per-cell advance, the reference kernel's recorded states."""
 import ctypes
 import os
+import time
 
 import numpy as np
 import pytest
@@ -19,9 +20,9 @@ def sms(gpu):
 
 
 @pytest.mark.parametrize("math", [0, 1])
-@pytest.mark.parametrize("tiles", [lambda sms: sms // 4, lambda sms: sms // 4 + 1, lambda sms: sms // 2,
-                                   lambda sms: sms // 2 + 1, lambda sms: sms + 3],
-                         ids=["cluster4", "cluster2", "cluster2_full", "block", "block_queue"])
+@pytest.mark.parametrize("tiles", [lambda sms: sms // 5, lambda sms: sms // 4, lambda sms: sms // 4 + 1,
+                                   lambda sms: sms // 2, lambda sms: sms // 2 + 1, lambda sms: sms + 3],
+                         ids=["four_blocks", "four_to_two", "two_blocks", "two_blocks_most", "one_block", "queue"])
 def test_cta32_shapes(wr, gpu, sms, oracle_port, tiles, math):
     """The structured policy on clusters of four blocks, of two, and on one block per tile
     (more tiles than SMs: blocks take a second one), the last tile ragged: three outer
@@ -49,7 +50,7 @@ def test_cta32_shapes(wr, gpu, sms, oracle_port, tiles, math):
 
     got, dts = steps(cells)
     assert got["stats"]["internal_steps"].sum() > got["stats"]["accepted_steps"].sum()  # rejected trials
-    for tile in (0, tiles(sms) // 2, tiles(sms) - 1):  # one tile: a cluster of four
+    for tile in (0, tiles(sms) // 2, tiles(sms) - 1):  # one tile: four blocks
         i = slice(32 * tile, 32 * tile + 32)
         assert steps(cells[i], dts)[0].tobytes() == got[i].tobytes()
     if math == wr.MATH_PORTABLE:
@@ -57,6 +58,30 @@ def test_cta32_shapes(wr, gpu, sms, oracle_port, tiles, math):
         rc, cgs = oracle_port.run_cta32(want, perturb=True, max_steps=3)
         assert rc == wr.SUCCESS and cgs == 3
         assert got.tobytes() == want.tobytes()
+
+
+def test_cta32_clusters_run_at_once(wr, gpu, sms):
+    """As long as there are two SMs per tile, a step of like tiles is one wave: a tile takes
+    1.4 times as long on two SMs as on four (measured), twice as long in two waves."""
+    def step(tiles):
+        cells = wr.make_grid(1).repeat(32 * tiles)
+        best = np.inf
+        with wr.Context(len(cells), 0, wr.MATH_PORTABLE) as ctx:
+            for _ in range(4):
+                ctx.set_policy(wr.POLICY_GRIDWIDE_INDEPENDENT)
+                ctx.upload(cells)
+                rc, dt = ctx.prepare(0, 0.0, 0, False)
+                assert rc == wr.SUCCESS
+                ctx.set_policy(wr.POLICY_GRIDWIDE_CTA32)
+                t = time.perf_counter()
+                rc, moved = ctx.advance(0, dt, dt)
+                best = min(best, time.perf_counter() - t)
+                assert rc == wr.SUCCESS and moved == len(cells)
+        return best
+
+    few = step(4)
+    for tiles in (sms // 4 - 1, sms // 4, sms // 2):
+        assert step(tiles) <= 1.7 * few, tiles
 
 
 @pytest.mark.parametrize("cells_of", [lambda sms: 1, lambda sms: 16 * sms, lambda sms: 16 * sms + 1,

@@ -75,27 +75,44 @@ cudaError_t WR_CAT(launch_advance_coop, WR_COOP_G)(int math_cuda, int blocks, cu
 // (wr_launch.h: cta32_shape picks the pair)
 namespace {
 template <class M, int CL>
-cudaError_t launch_cta32(int tiles, int sms, cudaStream_t stream, DevState s, StepCtl* ctl) {
-    constexpr size_t smem = static_cast<size_t>(kTileCells / CL) * Tab::kNV * 8;
-    static_assert(smem + sizeof(TileCtl<kTileCells / CL>) <= 232448, "a tile's block exceeds 227 KiB of shared memory");
-    auto k = k_advance_cta32<M, kG, CL, Tab>;
-    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(k), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
+struct Cta32Launch {
+    void (*kernel)(DevState, StepCtl*) = k_advance_cta32<M, kG, CL, Tab>;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(CL == 1 ? (tiles < sms ? tiles : sms) : tiles * CL));
-    cfg.blockDim = dim3(kTileCells / CL * kG);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
     cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = CL;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = CL > 1 ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, k, s, ctl);
+    cudaError_t configured;
+    explicit Cta32Launch(int blocks) {
+        constexpr size_t smem = static_cast<size_t>(kTileCells / CL) * Tab::kNV * 8;
+        static_assert(smem + sizeof(TileCtl<kTileCells / CL>) <= 232448,
+                      "a tile's block exceeds 227 KiB of shared memory");
+        configured = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+        cfg.blockDim = dim3(kTileCells / CL * kG);
+        cfg.dynamicSmemBytes = smem;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = CL;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = CL > 1 ? 1 : 0;
+    }
+    Cta32Launch(const Cta32Launch&) = delete;
+};
+template <class M, int CL>
+cudaError_t launch_cta32(int tiles, int sms, cudaStream_t stream, DevState s, StepCtl* ctl) {
+    Cta32Launch<M, CL> l(CL == 1 ? (tiles < sms ? tiles : sms) : tiles * CL);
+    if (l.configured != cudaSuccess) return l.configured;
+    l.cfg.stream = stream;
+    const cudaError_t e = cudaLaunchKernelEx(&l.cfg, l.kernel, s, ctl);
     return e == cudaSuccess ? cudaGetLastError() : e;
 }
+#if WR_COOP_G == 32
+template <class M, int CL>
+cudaError_t clusters_cta32(int* fit) {
+    Cta32Launch<M, CL> l(CL);
+    if (l.configured != cudaSuccess) return l.configured;
+    return cudaOccupancyMaxActiveClusters(fit, l.kernel, &l.cfg);
+}
+#endif
 }  // namespace
 #if WR_COOP_G != 8
 cudaError_t WR_CAT(launch_advance_cta32_, WR_COOP_G)(int math_cuda, int cluster, int tiles, int sms,
@@ -111,6 +128,12 @@ cudaError_t WR_CAT(launch_advance_cta32_, WR_COOP_G)(int math_cuda, int cluster,
     return math_cuda ? launch_cta32<CudaMath, 2>(tiles, sms, stream, s, ctl)
                      : launch_cta32<PortableMathCall, 2>(tiles, sms, stream, s, ctl);
 #endif
+}
+#endif
+#if WR_COOP_G == 32
+cudaError_t cta32_clusters(int math_cuda, int cluster, int* fit) {
+    if (cluster == 4) return math_cuda ? clusters_cta32<CudaMath, 4>(fit) : clusters_cta32<PortableMathCall, 4>(fit);
+    return math_cuda ? clusters_cta32<CudaMath, 2>(fit) : clusters_cta32<PortableMathCall, 2>(fit);
 }
 #endif
 

@@ -76,6 +76,7 @@ struct wr_ctx {
     unsigned long long* phases = nullptr;  // wr_diag_coop_phases: 16 device counters
     int policy = WR_POLICY_GRIDWIDE_INDEPENDENT;
     double* local_dt = nullptr;  // legacy-local policy: each cell's own dt
+    int cta32_fit[2] = {0, 0};   // cta32 policy: clusters of four and of two blocks that run at once
     cudaEvent_t ev[4 * WR_MAX_COLLAPSE_STEPS + 2] = {};
     int ev_used = 0;
     wr_run_timing timing{};
@@ -366,7 +367,7 @@ cudaError_t launch_advance(wr_ctx* ctx) {
     if (ctx->policy == WR_POLICY_GRIDWIDE_CTA32) {
         const int math_cuda = ctx->math == WR_MATH_CUDA ? 1 : 0;
         const int tiles = (ctx->n + 31) / 32;
-        const Cta32Shape sh = cta32_shape(tiles, ctx->sms);
+        const Cta32Shape sh = cta32_shape(tiles, ctx->cta32_fit[0], ctx->cta32_fit[1]);
         return sh.lanes == 16
                    ? launch_advance_cta32_16(math_cuda, sh.cluster, tiles, ctx->sms, ctx->stream, ctx->s, ctx->ctl)
                    : launch_advance_cta32_32(math_cuda, sh.cluster, tiles, ctx->sms, ctx->stream, ctx->s, ctx->ctl);
@@ -902,6 +903,12 @@ int wr_set_policy(wr_ctx* ctx, int policy) {
     if (policy == WR_POLICY_LEGACY_LOCAL && !ctx->local_dt) {
         const cudaError_t e = cudaMalloc(&ctx->local_dt, static_cast<size_t>(ctx->n) * sizeof(double));
         if (e != cudaSuccess) return fail("cudaMalloc(local dt)", e);
+    }
+    if (policy == WR_POLICY_GRIDWIDE_CTA32 && ctx->cta32_fit[1] == 0) {
+        const int math_cuda = ctx->math == WR_MATH_CUDA ? 1 : 0;
+        cudaError_t e = cta32_clusters(math_cuda, 4, &ctx->cta32_fit[0]);
+        if (e == cudaSuccess) e = cta32_clusters(math_cuda, 2, &ctx->cta32_fit[1]);
+        if (e != cudaSuccess) return fail("cta32 cluster occupancy", e);
     }
     ctx->policy = policy;
     ctx->s.local_dt = policy == WR_POLICY_LEGACY_LOCAL ? ctx->local_dt : nullptr;

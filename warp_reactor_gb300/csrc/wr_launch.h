@@ -65,13 +65,19 @@ cudaError_t configure_advance_portable();
 // gridwide-structured-cta32 policy (wr_coop_cta32.cuh): a tile of 32 cells on a cluster
 // of `cluster` SMs at `lanes` lanes per cell.  A trial's latency sets the time while
 // there are SMs to spare, so a tile spreads over four SMs (8 cells each) or two as long
-// as that takes no second wave; beyond that one SM per tile at 16 lanes per cell.
+// as the device runs all clusters at once; beyond that one SM per tile at 16 lanes per
+// cell.  fit4 and fit2 are the clusters that fit (cta32_clusters): the blocks of one lie
+// in one GPC, so of 152 SMs 36 clusters of four, not 38 (one outer step of like tiles:
+// up to 36 tiles 8.6 ms, 37 and 38 tiles 16.9 ms in two waves of them, 11.9 ms on
+// clusters of two, which take up to 76; from 77 on 15.2 ms on one SM per tile).
 struct Cta32Shape {
     int lanes, cluster;
 };
-constexpr Cta32Shape cta32_shape(int tiles, int sms) {
-    return tiles * 4 <= sms ? Cta32Shape{32, 4} : tiles * 2 <= sms ? Cta32Shape{32, 2} : Cta32Shape{16, 1};
+constexpr Cta32Shape cta32_shape(int tiles, int fit4, int fit2) {
+    return tiles <= fit4 ? Cta32Shape{32, 4} : tiles <= fit2 ? Cta32Shape{32, 2} : Cta32Shape{16, 1};
 }
+// clusters of 4 or 2 blocks of the 32-lane kernel that the current device runs at once
+cudaError_t cta32_clusters(int math_cuda, int cluster, int* fit);
 cudaError_t launch_advance_cta32_16(int math_cuda, int cluster, int tiles, int sms, cudaStream_t stream, DevState s,
                                     StepCtl* ctl);
 cudaError_t launch_advance_cta32_32(int math_cuda, int cluster, int tiles, int sms, cudaStream_t stream, DevState s,
