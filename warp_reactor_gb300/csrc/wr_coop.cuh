@@ -764,8 +764,8 @@ __device__ __forceinline__ int ros2s_attempt(uint64_t* V, const double (&y)[K], 
 // norm err: hnew from err alone, hgus with the Gustafsson factor.  Their two chains
 // (quotient, cube root, quotient, limits, quotient) run side by side, hnew's in the even
 // lanes and hgus's in the odd ones: one cube root and three quotients of latency instead
-// of two and five (a step of 20,011 cells in portable math 20.1 -> 19.8 ms, the structured
-// policy on 1,000 cells 89.2 -> 88.2 ms).  FMAX: limits by fmax and fmin (the structured
+// of two and five (a step of 20,011 cells in portable math 20.1 -> 19.5 ms, the structured
+// policy on 1,000 cells 89.2 -> 86.9 ms).  FMAX: limits by fmax and fmin (the structured
 // policy).
 template <int G, bool FMAX, class Cbrt>
 __device__ __forceinline__ void step_sizes(double err, double erracc, double hacc, double h, int gl, Cbrt cbrt,

@@ -18,7 +18,7 @@
 // anything else.  A tile's trials are serial, so with few tiles the time is a trial's
 // latency: 32 cells on one SM share its FP64 pipes, 8 cells on each of four SMs at 32
 // lanes per cell run a trial in half the time (the choice is cta32_shape's).  Measured
-// on GB300, 1,000 cells over the last eight outer steps of a collapse: 88 ms; one lane
+// on GB300, 1,000 cells over the last eight outer steps of a collapse: 87 ms; one lane
 // per cell and one warp per tile, as this kernel was before, 1,159 ms.
 #pragma once
 

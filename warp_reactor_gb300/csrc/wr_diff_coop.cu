@@ -16,7 +16,8 @@
 // One lane per cell, as these kernels were before, kept 128 warps of divergent lanes
 // and local-memory arrays on 152 SMs for 4,096 cells.  Measured on GB300 (forward and
 // adjoint of 4,096 cells over four outer steps, and of 64 cells over eight): 163 ms and
-// 566 ms before, 49 ms and 57 ms now, with the same bits.
+// 566 ms before, 47 ms and 50 ms now, with the same bits (at 65,536 cells over four outer
+// steps 296 + 892 ms before, 223 + 448 ms now).
 #include "generated/coop_diff.h"
 #include "wr_coop.cuh"
 #include "wr_diff.cuh"

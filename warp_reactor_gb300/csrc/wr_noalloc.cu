@@ -25,8 +25,8 @@
 // advance, whose matrices live in shared memory; the result equals wr_advance of a
 // WR_MATH_PORTABLE context bit for bit.  With at most 4,096 cells a call lasts as long
 // as its longest burn: the lane-per-cell advance, one FP64 instruction at a time for
-// a whole warp and its matrices in local memory, took 17.5 ms for a step of 1,000
-// cells, the cooperative one 2.6 ms.
+// a whole warp and its matrices in local memory, took 17.4 ms for a step of 1,000
+// cells, the cooperative one 2.3 ms.
 #include <cuda_runtime.h>
 
 #include <cstddef>

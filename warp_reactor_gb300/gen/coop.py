@@ -8,8 +8,9 @@ computes one node of the DAG from operands gathered out of ``V`` and stores it
 back into ``V``.  Between steps the warp
 synchronises, so a step may use any value produced by an earlier step.
 
-Step format (per lane, three 64-bit words; every address is the byte offset of a
-slot in the cell's own slot array, so the device adds it to one base):
+Step format of an encoded program (``encode``; per lane, three 64-bit words; every
+address is the byte offset of a slot in the cell's own slot array, so the device adds it
+to one base):
 
 * main word: four 16-bit fields X | Y | Z | D.  An FMA step computes
   ``V[D] = fma(V[X], V[Y] ^ L, V[Z])``; exp, log and sqrt take ``V[Y] ^ L`` and
@@ -28,9 +29,10 @@ slot in the cell's own slot array, so the device adds it to one base):
 * literal word L: the lane's constant operand, XOR-ed into ``V[Y]`` (``Y`` then
   names a slot holding +0.0, so the operand is the constant); 0 otherwise.
 
-The device's tables hold the same steps with plain addresses in X, Y and Z, the class
-and the step flags in a control byte per step (``device_words``), and the device
-overlaps neighbouring steps: a main result is read at the earliest ``MAIN_DELAY``
+The device does not read these flags: its tables (``device_words``) hold the same steps
+with plain addresses in X, Y and Z, the class and the step flags in a control byte per
+step and the argument modifiers in the low bits of D, and the device overlaps
+neighbouring steps: a main result is read at the earliest ``MAIN_DELAY``
 steps after its own.
 
 Constants therefore never need a table of their own: a network coefficient is the

@@ -1,5 +1,5 @@
 """Vector programs of the differentiation form, for the cooperative (lanes-per-cell)
-forward and adjoint kernels (csrc/wr_diff_coop.cuh).
+forward and adjoint kernels (csrc/wr_diff_coop.cu).
 
 The step format, scheduling and slot map are ``coop.py``'s.  The programs, for ``G`` = 32
 lanes per cell:
@@ -23,8 +23,9 @@ a select did not take may hold infinities, and 0 * inf must not reach the inputs
 (classes ``C_GMUL``, ``C_GDIV``) -- and products and sums round separately.  A stiff step's
 adjoint cancels ten digits and more, so another order of the same sums would give
 gradients that agree with the straight-line code's to six digits only, no better and no
-worse; this one gives the same bits.  (The price is the serial sum of the contributions to
-T and log T, several hundred for the Jacobian: it is the program's critical path.)
+worse; this one gives the same bits (a zero may have the other sign).  (The price is the
+serial sum of the contributions to T and log T, several hundred for the Jacobian: it is
+the program's critical path.)
 
 Slots: the multipliers and fbar have reserved slots above the constants; no program
 writes them, nor the matrix slots but for ``jrhsp``.
@@ -73,7 +74,6 @@ TUNE = {
     ("rhsvjp", 6): ((1.5, 5.0, 66987, 0.1, 30), 1800),
     ("jacvjp", 6): ((6.0, None, 701470, 0.01, 30), 1500),
 }
-DEFAULT_TUNE = ((3.0, None, 1, 0.01, 20), None)
 
 
 def prologue(P: Program):
@@ -256,7 +256,7 @@ def generate(regimes=REGIMES, tune=TUNE) -> dict:
     first = RES_BASE + len(keys)
     scheds = {}
     for (kind, r), (P, out) in built.items():
-        t, lim = tune.get((kind, r), tune.get(kind, DEFAULT_TUNE))
+        t, lim = tune[kind, r]
         scheds[kind, r] = schedule(P, out, G, jac=kind == "jrhsp", limit=lim, first_scratch=first, tune=t)[0]
     # two sizes of the slot array: the forward kernel holds the first alone
     fwd = max(s.nv for (kind, _), s in scheds.items() if kind in ("jrhsp", "rhsp"))
