@@ -24,7 +24,8 @@ PTX = {
 
 def compile_program(tmp, name, parts):
     """``name``.cpp with the device code ``parts`` as device_code.h, under the sanitizer."""
-    for header in ("wr_coop.cuh", "wr_kernels.cuh", "wr_physics.cuh", "wr_math.h", "wr_diff.cuh"):
+    for header in ("wr_coop.cuh", "wr_kernels.cuh", "wr_physics.cuh", "wr_math.h", "wr_diff.cuh",
+                   "wr_coop_cta32.cuh"):
         src = open(os.path.join(CSRC, header)).read().replace('"../../include/', f'"{INCLUDE}/')
         if header == "wr_coop.cuh":
             for asm, cxx in PTX.items():
@@ -35,11 +36,17 @@ def compile_program(tmp, name, parts):
             host = "#else\n    return a / b;\n#endif"
             assert src.count(host) == 1
             src = src.replace(host, host.replace("a / b", "native_division(a, b)"))
+        # shared by the block, once: its dynamic shared memory is the program's array sm
+        src = re.sub(r"(?<!extern )__shared__ ", "static ", src)
         (tmp / header).write_text(src)
     (tmp / "cuda_runtime.h").write_text("#pragma once\nusing cudaError_t = int;\nusing cudaStream_t = void*;\n")
+    (tmp / "cooperative_groups.h").write_text(
+        "#pragma once\nnamespace cooperative_groups {\nstruct cluster_group {\n    void sync() {}\n"
+        "    template <class T>\n    T* map_shared_rank(T* p, int) { return p; }\n};\n"
+        "inline cluster_group this_cluster() { return {}; }\n}\n")
     (tmp / "device_code.h").write_text(parts)
     exe = str(tmp / name)
-    r = subprocess.run(["g++", "-std=c++17", "-O1", "-g", "-fsanitize=thread", "-ffp-contract=off", "-Wno-unknown-pragmas",
+    r = subprocess.run(["g++", "-std=c++20", "-O1", "-g", "-fsanitize=thread", "-ffp-contract=off", "-Wno-unknown-pragmas",
                         "-I", str(tmp), "-I", HERE, "-I", CSRC, os.path.join(HERE, name + ".cpp"), "-o", exe, "-pthread"],
                        capture_output=True, text=True)
     if "tsan" in r.stderr and "cannot find" in r.stderr:
@@ -59,15 +66,19 @@ def run_program(exe, *args):
     return r.stdout
 
 
-@pytest.fixture(scope="module", params=[8, 16, 32])
-def advance(request, built, tmp_path_factory):
-    G = request.param
+def advance_tables(G):
+    """The tables of G lanes per cell as wr_adv_coop.cuh presents them to the kernels."""
     unit = open(os.path.join(CSRC, "wr_adv_coop.cuh")).read()
     tables = unit[unit.index("namespace cp ="):unit.index("static_assert(coop::kRes")].replace(
         "WR_CAT(coop, WR_COOP_G)", f"coop{G}").replace("int first(int w) { ", "int first(int w) { started(w); ")
     assert "started" in tables
-    parts = f'#include "generated/coop_prog_g{G}.h"\n#include "wr_coop.cuh"\nnamespace wr {{\n{tables}\n}}\n'
-    return compile_program(tmp_path_factory.mktemp(f"advance{G}"), "advance", parts)
+    return f'#include "generated/coop_prog_g{G}.h"\n#include "wr_coop.cuh"\nnamespace wr {{\n{tables}\n}}\n'
+
+
+@pytest.fixture(scope="module", params=[8, 16, 32])
+def advance(request, built, tmp_path_factory):
+    parts = advance_tables(request.param)
+    return compile_program(tmp_path_factory.mktemp(f"advance{request.param}"), "advance", parts)
 
 
 def burn(advance, tmp, oracle, wr, cells, dt):
@@ -110,6 +121,28 @@ def test_group_without_cell_follows(advance, tmp_path, oracle_port, wr, order):
     else:
         want = programs[:3] + alone[:1] + alone[3:]
     assert programs == want
+
+
+@pytest.fixture(scope="module")
+def tiles(built, tmp_path_factory):
+    parts = "inline void started(int) {}\n" + advance_tables(16) + '#include "wr_coop_cta32.cuh"\n'
+    return compile_program(tmp_path_factory.mktemp("tiles"), "tiles", parts)
+
+
+def test_tiles(tiles, tmp_path, oracle_port, wr):
+    """The structured policy's block: 16 warps, a full tile and a ragged one after it, whose
+    trials one warp decides; some warps of the second hold one cell, most none."""
+    cells = np.tile(wr.make_batch_grid(1, 35, log10_tmin=2.5, log10_tmax=3.2)[32:], 12)[:35]  # few trials
+    want = cells.copy()
+    rc, dt = oracle_port.prepare(cells.copy(), 0, 0.0, 0, True)
+    assert rc == wr.SUCCESS
+    rc, cgs = oracle_port.run_cta32(want, perturb=True, max_steps=1)
+    assert (rc, cgs) == (wr.SUCCESS, 1)
+    assert want["stats"]["internal_steps"].sum() > want["stats"]["accepted_steps"].sum()  # rejected trials
+    (tmp_path / "in").write_bytes(cells.tobytes())
+    out = run_program(tiles, dt, tmp_path / "in", tmp_path / "out")
+    assert [int(v) for v in out.split()] == [wr.SUCCESS, len(cells)]
+    assert (tmp_path / "out").read_bytes() == want.tobytes()
 
 
 @pytest.fixture(scope="module")

@@ -1,18 +1,16 @@
-// warp_threads.h -- a warp on the CPU: one thread per lane, for compiling the device
+// warp_threads.h -- a block on the CPU: one thread per lane, for compiling the device
 // code of csrc/*.cuh with the host compiler and running it under ThreadSanitizer.
 //
-// What orders memory here is what orders it on the device: __syncwarp (a barrier that
-// the sanitizer sees) orders the lanes' accesses before it against those after it;
-// shuffles and votes exchange values but order nothing (the sanitizer is told to ignore
-// their synchronisation).  So two lanes' accesses to one word of the slot array, one of
-// them a write, with no __syncwarp between them, are a reported race whatever order the
-// threads happened to run in.
+// What orders memory here is what orders it on the device: __syncwarp and __syncthreads
+// (barriers that the sanitizer sees) order the lanes' accesses before them against those
+// after them; shuffles and votes exchange values but order nothing (the sanitizer is told
+// to ignore their synchronisation).  So two lanes' accesses to one word of shared memory,
+// one of them a write, with no barrier between them, are a reported race whatever order
+// the threads happened to run in.
 //
-// The one-warp launch has threadIdx.x = lane; warp-collective calls take any lane mask
-// (groups of a warp diverge in the advance's queue loop).
+// Warp-collective calls take any lane mask (groups of a warp diverge in the advance's
+// queue loop).
 #pragma once
-
-#include <sched.h>
 
 #include <algorithm>
 #include <atomic>
@@ -71,18 +69,22 @@ struct Meeting {
         if (arrived.fetch_add(1, std::memory_order_acq_rel) + 1 == static_cast<unsigned>(lanes)) {
             arrived.store(0, std::memory_order_relaxed);
             turn.store(t + 1, std::memory_order_release);
+            turn.notify_all();
         } else {
-            while (turn.load(std::memory_order_acquire) == t) sched_yield();
+            turn.wait(t, std::memory_order_acquire);
         }
         return get(word[t & 1]);
     }
 };
-// one per group of lanes (a mask is a run of lanes whose first and size identify it)
-inline Meeting meetings[6][kLanes];
+// one per warp and group of lanes (a mask is a run of lanes whose first and size identify it)
+constexpr int kWarps = 16;
+inline Meeting meetings[kWarps][6][kLanes];
 inline Meeting& meeting(unsigned mask) {
-    return meetings[__builtin_ctz(static_cast<unsigned>(__builtin_popcount(mask)))][__builtin_ctz(mask)];
+    return meetings[threadIdx.x / kLanes][__builtin_ctz(static_cast<unsigned>(__builtin_popcount(mask)))]
+                   [__builtin_ctz(mask)];
 }
-inline int lane() { return static_cast<int>(threadIdx.x); }
+inline Meeting block;  // of all threads: word[.][0] is unused
+inline int lane() { return static_cast<int>(threadIdx.x % kLanes); }
 
 struct IgnoreSync {
     IgnoreSync() { AnnotateIgnoreSyncBegin(__FILE__, __LINE__); }
@@ -110,10 +112,11 @@ T exchange(unsigned mask, T v, int from) {  // the value of lane `from`
     }));
 }
 
-// a kernel's body on the 32 lanes of one warp
-inline void launch(const std::function<void()>& body) {
+// a kernel's body on one block of `warps` warps
+inline void launch(const std::function<void()>& body, int warps = 1) {
+    blockDim.x = static_cast<unsigned>(warps * kLanes);
     std::vector<std::thread> lanes;
-    for (int l = 0; l < kLanes; ++l)
+    for (int l = 0; l < warps * kLanes; ++l)
         lanes.emplace_back([l, &body] {
             threadIdx.x = static_cast<unsigned>(l);
             body();
@@ -177,7 +180,10 @@ using std::isfinite;
 inline unsigned min(unsigned a, int b) { return std::min(a, static_cast<unsigned>(b)); }
 inline int __popc(unsigned v) { return __builtin_popcount(v); }
 inline int __ffs(unsigned v) { return v ? __builtin_ctz(v) + 1 : 0; }
-inline void __syncthreads() { __syncwarp(); }
+inline void __syncthreads() {
+    warp::block.meet(0, warp::lane(), static_cast<int>(blockDim.x), [](const auto*) { return uint64_t{0}; });
+    ++warp::step;
+}
 
 inline double __longlong_as_double(long long v) { return warp::from_word<double>(static_cast<uint64_t>(v)); }
 inline long long __double_as_longlong(double v) { return static_cast<long long>(warp::to_word(v)); }
